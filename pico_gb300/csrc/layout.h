@@ -43,13 +43,12 @@ PICO_HD bool pico_is_leaf(uint32_t ref) { return (ref & PICO_REF_LEAF) != 0u; }
 PICO_HD uint32_t pico_leaf_first(uint32_t ref) { return (ref & 0x7fffffffu) >> 5; }
 PICO_HD uint32_t pico_leaf_count(uint32_t ref) { return ref & 31u; }
 
-struct alignas(16) GpuNode {
-    float c0lox, c0hix, c0loy, c0hiy;
-    float c1lox, c1hix, c1loy, c1hiy;
+struct alignas(32) GpuNode {
+    float c0lox, c0loy, c0hix, c0hiy, c1lox, c1loy, c1hix, c1hiy;
     float c0loz, c0hiz, c1loz, c1hiz;
     uint32_t ref0, ref1, pad0, pad1;
 };
-static_assert(sizeof(GpuNode) == 64, "node is one 64-byte record");
+static_assert(sizeof(GpuNode) == 64, "node is two 32-byte loads");
 
 struct alignas(16) GpuTri {
     float v0x, v0y, v0z; uint32_t prim;
