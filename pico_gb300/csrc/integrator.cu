@@ -230,14 +230,12 @@ struct ExtendRays {
 // (they write disjoint path fields and both finish before the next shade), so a
 // depth pays one launch and one tail.  kThreads per CTA (64, 128 or 256): the
 // block shape batched renders tune; the register budget is the same for every
-// shape: 1024 threads (64 registers) per SM in the near-first order, where against
-// 896 threads at 72 registers the 1080p renders measured 2 % faster with identical
-// images (the extra warps hide more latency than the few spilled registers cost),
-// and 896 threads in the reference's order, which spills more at 64.  kCount: the
-// same traversal, also adding its work (nodes, triangles, instance entries) to
-// `counters` (measurement only).
+// shape: 1152 threads (56 registers) per SM in the near-first order (walk_queue gives
+// the figures), and 896 threads in the reference's order, which spills more at 64.
+// kCount: the same traversal, also adding its work (nodes, triangles, instance
+// entries) to `counters` (measurement only).
 template <int kOrder>
-constexpr int extend_threads_per_sm() { return (kOrder & kReferenceOrder) ? 896 : 1024; }
+constexpr int extend_threads_per_sm() { return (kOrder & kReferenceOrder) ? 896 : 1152; }
 template <int kOrder, int kThreads, bool kCount = false>
 __global__ void __launch_bounds__(kThreads, extend_threads_per_sm<kOrder>() / kThreads) extend_kernel(SceneView sc, PathBatch b, const uint32_t* q,
                                                        const uint32_t* count, const uint32_t* sq,
@@ -869,18 +867,33 @@ __global__ void __launch_bounds__(kRenderThreads) prepare_image_kernel(const uin
 }
 
 // Scene::generate_denoiser_inputs: one primary ray per pixel with xi = (0, 0).
-template <int kOrder>
-__global__ void __launch_bounds__(128) gbuffer_kernel(SceneView sc, CameraView cam, uint32_t W, uint32_t H,
-                                                     float* normals, float* positions, float* diffuse, int* err)
-{
-    using namespace ex;
-    const uint32_t npx = W * H;
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += gridDim.x * blockDim.x) {
+struct GbufferRays {
+    using Tag = uint32_t;
+    using Index = uint64_t;
+    const SceneView& sc;
+    const CameraView& cam;
+    uint32_t W;
+    float* normals;
+    float* positions;
+    float* diffuse;
+    int* err;
+
+    __device__ __forceinline__ uint32_t load(uint64_t k, float4& o, float4& d, float& tmax, float& exit_below,
+                                             bool& occlusion) const
+    {
+        camera_ray(cam, 0.0f, 0.0f, (uint32_t)k % W, (uint32_t)k / W, o, d);
+        tmax = INFINITY;
+        exit_below = -INFINITY;
+        occlusion = false;
+        return (uint32_t)k;
+    }
+
+    __device__ __forceinline__ void finish(uint32_t p, const TraceHit& h, int s) const
+    {
+        using namespace ex;
+        if (s != kTraceOk) atomicOr(err, s);
         float4 o, d;
         camera_ray(cam, 0.0f, 0.0f, p % W, p / W, o, d);
-        TraceHit h;
-        const int s = trace_closest<false, kOrder>(sc, o, d, h, nullptr);
-        if (s != kTraceOk) atomicOr(err, s);
         float n[3], pos[3], alb[3];
         if (s == kTraceOk && h.rank != kNoHit) {
             const Fragment f = make_fragment(sc, h.rank, h.tri, h.u, h.v, o, d);
@@ -901,6 +914,30 @@ __global__ void __launch_bounds__(128) gbuffer_kernel(SceneView sc, CameraView c
             normals[3 * (size_t)p + c] = n[c];
             positions[3 * (size_t)p + c] = pos[c];
             diffuse[3 * (size_t)p + c] = alb[c];
+        }
+    }
+};
+
+template <int kOrder>
+__global__ void __launch_bounds__(128) gbuffer_kernel(SceneView sc, CameraView cam, uint32_t W, uint32_t H,
+                                                     float* normals, float* positions, float* diffuse,
+                                                     unsigned long long* work, int* err)
+{
+    GbufferRays rays{sc, cam, W, normals, positions, diffuse, err};
+    const uint64_t npx = (uint64_t)W * H;
+    if constexpr ((kOrder & kReferenceOrder) == 0) {
+        TraceCounters cnt{0, 0, 0, 0};
+        walk_queue<false, (kOrder & kWithImplicit) != 0, (kOrder & kBounded) != 0, (kOrder & kWatertight) != 0>(
+            sc, rays, npx, work, &cnt);
+    } else {
+        for (uint64_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += gridDim.x * blockDim.x) {
+            float4 o, d;
+            float tmax, exit_below;
+            bool occlusion;
+            const uint32_t tag = rays.load(p, o, d, tmax, exit_below, occlusion);
+            TraceHit h;
+            const int s = trace_closest<false, kOrder>(sc, o, d, h, nullptr);
+            rays.finish(tag, h, s);
         }
     }
 }
@@ -1126,9 +1163,12 @@ cudaError_t launch_prepare_image(const uint32_t* count, uint32_t npx, uint32_t m
 cudaError_t launch_gbuffer(const SceneView& sc, const CameraView& cam, uint32_t W, uint32_t H, float* normals,
                            float* positions, float* diffuse, DeviceStatus* status, int order, cudaStream_t st)
 {
+    const cudaError_t e = cudaMemsetAsync(&status->work, 0, sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
     with_variant(order, sc, [&](auto v) {
-        gbuffer_kernel<decltype(v)::value><<<grid_for(gbuffer_kernel<decltype(v)::value>, W * H, 128), 128, 0, st>>>(sc, cam, W, H, normals, positions,
-                                                                                 diffuse, &status->trace_error);
+        constexpr int V = decltype(v)::value;
+        gbuffer_kernel<V><<<grid_for(gbuffer_kernel<V>, W * H, 128), 128, 0, st>>>(
+            sc, cam, W, H, normals, positions, diffuse, &status->work, &status->trace_error);
     });
     return cudaGetLastError();
 }

@@ -711,12 +711,13 @@ std::string build_flat_scene(const pico_scene_desc& desc, FlatScene& fs)
         BinnedSahBuilder(refit).build(titems);
     }
     auto list_ranks = [&](const std::vector<uint32_t>& ranks) -> uint32_t {
+        if (ranks.size() == 1) return ranks[0];   // items [0, ninstances) are the ranks themselves
         const uint32_t first = (uint32_t)fs.tlas_items.size();
         fs.tlas_items.insert(fs.tlas_items.end(), ranks.begin(), ranks.end());
         return first;
     };
     fs.tlas_fast_root_ref = flatten(refit, fs.nodes, list_ranks);
-    if (fs.tlas_items.size() > PICO_FIRST_MAX) return "too many instances";
+    if (2 * (uint64_t)desc.ninstances > PICO_FIRST_MAX) return "too many instances";
     if (refit.root != kInvalid) {
         const Box& b = refit.nodes[refit.root].box;
         fs.tlas_fast_lo[0] = b.lo.x; fs.tlas_fast_lo[1] = b.lo.y; fs.tlas_fast_lo[2] = b.lo.z;

@@ -4,10 +4,9 @@
 // Persistent: the grid is a whole number of CTAs per SM and the warps pull rays
 // from a global counter, so long rays do not leave SMs idle at the tail of the
 // batch.  In the near-first order a warp's lanes walk the batch with
-// walk_queue: one ballot per move decides whether the rarer moves wait, and
-// idle lanes take new rays in batches; in the reference order each warp takes
-// 32 rays at a time and each lane runs its ray to completion.  128 threads with
-// at most 64 registers each keep eight CTAs resident per SM.  Rays are 32 B
+// walk_queue; in the reference order each warp takes 32 rays at a time and each
+// lane runs its ray to completion.  128 threads with at most 56 registers each
+// keep nine CTAs resident per SM (walk_queue gives the figures).  Rays are 32 B
 // (two 16-byte loads), hits 20 B.
 #include "kernels.h"
 #include "traverse.cuh"
@@ -19,7 +18,9 @@
 namespace pico {
 
 constexpr int kTraceThreads = 128;
-constexpr int kTraceMinBlocks = 8;
+// CTAs per SM the kernel is compiled for: 56 registers for the near-first walk, 64 for the reference order.
+template <int kOrder>
+constexpr int trace_min_blocks() { return (kOrder & kReferenceOrder) ? 8 : 9; }
 
 __device__ __forceinline__ void write_hit(const SceneView& sc, const TraceHit& h, int s, pico_hit* out)
 {
@@ -63,7 +64,7 @@ struct BatchRays {
 };
 
 template <bool kCount, int kOrder>
-__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
+__global__ void __launch_bounds__(kTraceThreads, trace_min_blocks<kOrder>())
     trace_kernel(SceneView sc, const float4* __restrict__ rays, uint64_t n, pico_hit* __restrict__ hits,
                  DeviceStatus* status)
 {

@@ -408,8 +408,15 @@ __device__ __forceinline__ float world_distance(const SceneView& sc, uint32_t ra
     return world_distance_at(sc, rank, px, py, pz, o);
 }
 
-// The state of one near-first walk (the traversal stack is kept apart, in the
-// caller's local array, so that the state itself can live in registers).
+// The instance of a TLAS item.  The first ninstances items are the ranks themselves (the reference tree's), and a
+// near-first leaf of one instance names its rank directly, so the list is read for shared near-first leaves alone.
+__device__ __forceinline__ uint32_t tlas_rank(const SceneView& sc, uint32_t item)
+{
+    return item < sc.ninstances ? item : __ldg(sc.tlas_items + item);
+}
+
+// The state of one near-first walk.  What the inner-node moves use lives in registers; what only the rarer moves
+// use lives in the walk's local memory, behind its stack (WalkMemory), which keeps the kernels free of spills.
 //
 // The ray the node tests use is the world ray in the TLAS and the object-space
 // ray inside an instance, switched on entering and leaving an instance.  `limit`
@@ -417,36 +424,53 @@ __device__ __forceinline__ float world_distance(const SceneView& sc, uint32_t ra
 // TLAS, min(object-space best, BLAS bound) inside), clamped to the largest
 // finite float so that one comparison also rejects boxes at +inf.
 struct NearFirstState {
-    float4 o, d;                     // the world ray
-    TraceHit best;
-    float exit_below;                // the walk ends once its best hit lies below this
     float nx, ny, nz, cix, ciy, ciz; // the current level's ray: minus its origin, and its reciprocals
     float wmag, cmag;                // the watertight box slack's origin term (world, current)
     float limit;
     float qdx, qdy, qdz;             // object-space direction of the instance being searched
-    float lt, lu, lv;                // the instance's best triangle so far (object-space t)
-    uint32_t ltri, cur, ref, iter;
+    float lt;                        // the instance's best triangle so far: its object-space t
+    uint32_t ref, iter;
     int sp;
     bool wfast, cfast, in_blas;
 };
 
+// Per-lane local memory of a walk: the stack, then the fields of the rarer moves.
+enum WalkMemory : int {
+    kMemO = kTraceStack,             // the world ray's origin (4) and direction (3)
+    kMemD = kMemO + 4,
+    kMemR = kMemD + 3,               // the direction's reciprocals (3)
+    kMemExit = kMemR + 3,            // the walk ends once its best hit lies below this
+    kMemT, kMemRank, kMemTri,        // the best hit so far: distance, instance rank, triangle,
+    kMemU, kMemV,                    // barycentrics (an implicit hit's object-space t)
+    kMemCur, kMemLtri,               // the instance being searched, its best triangle so far (slot)
+    kMemLu, kMemLv,                  // and its barycentrics
+    kMemWords
+};
+__device__ __forceinline__ float mem_float(const uint32_t* mem, int k) { return __uint_as_float(mem[k]); }
+__device__ __forceinline__ void mem_set(uint32_t* mem, int k, float v) { mem[k] = __float_as_uint(v); }
+
 // Sets a walk up.  tmax bounds the hits that count; `occlusion` gives the
 // occlusion query: only hits strictly below tmax count (best starts at (tmax,
 // rank 0), so no candidate ties it) and the walk ends at the first instance
-// whose candidate is one, reported as best.tri != kNoHit.  Otherwise the walk
+// whose candidate is one, reported as a triangle other than kNoHit.  Otherwise the walk
 // ends early once its best hit lies below exit_below: the closest hit then lies
 // below it too, and a caller that only asks what kind of instance is hit (a
 // shadow ray whose lights all lie at or beyond exit_below) has its answer.
 template <bool kWT>
-__device__ __forceinline__ void nf_start(NearFirstState& w, const SceneView& sc, const float4 o, const float4 d,
-                                         float tmax, float exit_below, bool occlusion)
+__device__ __forceinline__ void nf_start(NearFirstState& w, uint32_t* mem, const SceneView& sc, const float4 o,
+                                         const float4 d, float tmax, float exit_below, bool occlusion)
 {
     const float kInf = __int_as_float(0x7f800000);
     const float kMaxFinite = __int_as_float(0x7f7fffff);
-    w.o = o; w.d = d;
-    w.best.t = tmax; w.best.rank = occlusion ? 0u : kNoHit; w.best.tri = kNoHit; w.best.u = 0.0f; w.best.v = 0.0f;
-    w.exit_below = occlusion ? kInf : exit_below;
+    mem_set(mem, kMemO, o.x); mem_set(mem, kMemO + 1, o.y); mem_set(mem, kMemO + 2, o.z); mem_set(mem, kMemO + 3, o.w);
+    mem_set(mem, kMemD, d.x); mem_set(mem, kMemD + 1, d.y); mem_set(mem, kMemD + 2, d.z);
+    mem_set(mem, kMemT, tmax);
+    mem[kMemRank] = occlusion ? 0u : kNoHit;
+    mem[kMemTri] = kNoHit;
+    mem[kMemU] = 0u; mem[kMemV] = 0u;
+    mem_set(mem, kMemExit, occlusion ? kInf : exit_below);
     const float wix = __frcp_rn(d.x), wiy = __frcp_rn(d.y), wiz = __frcp_rn(d.z);
+    mem_set(mem, kMemR, wix); mem_set(mem, kMemR + 1, wiy); mem_set(mem, kMemR + 2, wiz);
     // node tests take the NaN-free form when the ray (world or object space) and the boxes are finite
     w.wfast = sc.finite_boxes && all_finite(o.x, o.y, o.z, wix, wiy, wiz);
     w.nx = -o.x; w.ny = -o.y; w.nz = -o.z; w.cix = wix; w.ciy = wiy; w.ciz = wiz;
@@ -455,8 +479,7 @@ __device__ __forceinline__ void nf_start(NearFirstState& w, const SceneView& sc,
     w.cmag = w.wmag;
     w.limit = fminf(tmax, kMaxFinite);
     w.qdx = 0.0f; w.qdy = 0.0f; w.qdz = 0.0f;
-    w.lt = kInf; w.lu = 0.0f; w.lv = 0.0f;
-    w.ltri = kNoHit; w.cur = 0; w.iter = 0; w.sp = 0;
+    w.lt = kInf; w.iter = 0; w.sp = 0;
     w.in_blas = false;
     // A ray with a zero direction component whose origin lies on a box plane gets
     // a NaN slab distance there, and the reference skips that box.  Such rays walk
@@ -475,224 +498,256 @@ __device__ __forceinline__ void nf_start(NearFirstState& w, const SceneView& sc,
     if (h && tm < kInf) w.ref = axis ? sc.tlas_root_ref : sc.tlas_fast_root_ref;
 }
 
-// One move of a walk: an inner node, a BLAS leaf, an instance entry or an
-// instance exit.  Returns -1 while the walk goes on, else its final status
-// (kTraceOk, or the code of the bound it ran into).  One exit at the end: the
-// form with a return per case made the renders 2.4 % slower.
-template <bool kCount, bool kImplicit, bool kRuntimeBounds, bool kWT>
-__device__ __forceinline__ int nf_move(NearFirstState& w, const SceneView& sc, uint32_t* stack, TraceCounters* cnt)
+// What a walk is doing: its next move (kWalking), nothing (kIdle), or waiting to hand in its result with this
+// TraceStatus (>= 0).
+constexpr int kWalking = -1, kIdle = -2;
+
+__device__ __forceinline__ float4 nf_origin(const uint32_t* mem)
 {
-    using namespace ex;
-    const uint32_t max_iter = kRuntimeBounds ? sc.max_iterations : kTraceMaxIter;
+    return make_float4(mem_float(mem, kMemO), mem_float(mem, kMemO + 1), mem_float(mem, kMemO + 2),
+                       mem_float(mem, kMemO + 3));
+}
+__device__ __forceinline__ void nf_pop(NearFirstState& w, const uint32_t* mem)
+{
+    w.ref = w.sp ? mem[--w.sp] : PICO_REF_DONE;
+}
+
+// An inner node: both children tested, the nearer one next, the other on the stack.
+template <bool kCount, bool kRuntimeBounds, bool kWT>
+__device__ __forceinline__ int nf_inner(NearFirstState& w, const SceneView& sc, uint32_t* mem, TraceCounters* cnt)
+{
+    const int max_stack = kRuntimeBounds ? (int)sc.stack_entries : kTraceStack;
+    if (kRuntimeBounds && w.iter >= sc.max_iterations) return kTraceIterLimit;
+    ++w.iter;
+    float p[8], q[8];
+    load256(sc.nodes + w.ref, p);
+    load256(reinterpret_cast<const char*>(sc.nodes + w.ref) + 32, q);
+    const uint32_t ref0 = __float_as_uint(q[4]), ref1 = __float_as_uint(q[5]);
+    if (kCount) {
+        cnt->nodes++;
+        if (w.in_blas) cnt->blas_nodes++;
+    }
+    bool h0, h1;
+    float t0, t1;
+    if constexpr (kWT) {
+        t0 = slab_robust(p[0], p[2], p[1], p[3], q[0], q[1], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, w.cmag, h0);
+        t1 = slab_robust(p[4], p[6], p[5], p[7], q[2], q[3], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, w.cmag, h1);
+    } else if (w.cfast) {
+        const float2 nxy = make_float2(w.nx, w.ny), nzz = make_float2(w.nz, w.nz);
+        const float2 ixy = make_float2(w.cix, w.ciy), izz = make_float2(w.ciz, w.ciz);
+        t0 = slab_pairs(make_float2(p[0], p[1]), make_float2(p[2], p[3]), make_float2(q[0], q[1]), nxy, nzz, ixy, izz,
+                        h0);
+        t1 = slab_pairs(make_float2(p[4], p[5]), make_float2(p[6], p[7]), make_float2(q[2], q[3]), nxy, nzz, ixy, izz,
+                        h1);
+    } else {
+        t0 = slab(p[0], p[2], p[1], p[3], q[0], q[1], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, h0);
+        t1 = slab(p[4], p[6], p[5], p[7], q[2], q[3], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, h1);
+    }
+    // t <= limit (finite) also rejects t = +inf and NaN, like "t <= best && t < inf"
+    const bool v0 = h0 && t0 <= w.limit;
+    const bool v1 = h1 && t1 <= w.limit;
+    int status = kWalking;
+    if (v0 && v1) {
+        const bool swap = t1 < t0;
+        if (w.sp >= max_stack) {
+            status = kTraceStackOverflow;
+        } else {
+            mem[w.sp++] = swap ? ref0 : ref1;
+            w.ref = swap ? ref1 : ref0;
+        }
+    } else if (v0) {
+        w.ref = ref0;
+    } else if (v1) {
+        w.ref = ref1;
+    } else {
+        nf_pop(w, mem);
+    }
+    return status;
+}
+
+// A BLAS leaf's triangles.
+template <bool kCount, bool kWT>
+__device__ __forceinline__ void nf_leaf(NearFirstState& w, const SceneView& sc, uint32_t* mem, TraceCounters* cnt)
+{
+    ++w.iter;
+    const uint32_t first = pico_leaf_first(w.ref), end = first + pico_leaf_count(w.ref);
+    uint32_t ltri = mem[kMemLtri];
+    for (uint32_t tri = first; tri < end; ++tri) {
+        float t, u, v;
+        if (kCount) cnt->tris++;
+        if (intersect<kWT>(sc.tris + tri, -w.nx, -w.ny, -w.nz, w.qdx, w.qdy, w.qdz, t, u, v) &&
+            (t < w.lt || (t == w.lt && tri < ltri))) {
+            w.lt = t;
+            ltri = tri;
+            mem[kMemLtri] = tri;
+            mem_set(mem, kMemLu, u); mem_set(mem, kMemLv, v);
+        }
+    }
+    w.limit = fminf(w.limit, w.lt);
+    nf_pop(w, mem);
+}
+
+// A candidate (world distance tw on instance `rank`) against the best hit: the nearer one, of equal ones the lower
+// rank.  True when the walk may end with it.
+__device__ __forceinline__ bool nf_candidate(uint32_t* mem, float tw, uint32_t rank, uint32_t tri,
+                                             float u, float v)
+{
+    const float best = mem_float(mem, kMemT);
+    if (!(tw < best || (tw == best && rank < mem[kMemRank]))) return false;
+    mem_set(mem, kMemT, tw);
+    mem[kMemRank] = rank;
+    mem[kMemTri] = tri;
+    mem_set(mem, kMemU, u); mem_set(mem, kMemV, v);
+    return tw < mem_float(mem, kMemExit);
+}
+
+// Leaves an instance: its candidate is the closest triangle by object-space t.  Back to the world ray.
+__device__ __forceinline__ int nf_exit(NearFirstState& w, const SceneView& sc, uint32_t* mem)
+{
+    ++w.iter;
+    int status = kWalking;
+    const float4 o = nf_origin(mem);
+    const uint32_t ltri = mem[kMemLtri];
+    if (ltri != kNoHit) {
+        const uint32_t cur = mem[kMemCur];
+        const float lu = mem_float(mem, kMemLu), lv = mem_float(mem, kMemLv);
+        const float tw = world_distance(sc, cur, ltri, lu, lv, o);
+        if (nf_candidate(mem, tw, cur, ltri, lu, lv)) status = kTraceOk;
+    }
+    w.in_blas = false;
+    w.nx = -o.x; w.ny = -o.y; w.nz = -o.z;
+    w.cix = mem_float(mem, kMemR); w.ciy = mem_float(mem, kMemR + 1); w.ciz = mem_float(mem, kMemR + 2);
+    w.cfast = w.wfast;
+    w.cmag = w.wmag;
+    w.limit = fminf(mem_float(mem, kMemT), __int_as_float(0x7f7fffff));
+    nf_pop(w, mem);
+    return status;
+}
+
+// A TLAS leaf: searches the instance of its first item; the rest of the leaf waits on the stack.
+template <bool kCount, bool kImplicit, bool kRuntimeBounds, bool kWT>
+__device__ __forceinline__ int nf_enter(NearFirstState& w, const SceneView& sc, uint32_t* mem, TraceCounters* cnt)
+{
     const int max_stack = kRuntimeBounds ? (int)sc.stack_entries : kTraceStack;
     const float kInf = __int_as_float(0x7f800000);
     const float kMaxFinite = __int_as_float(0x7f7fffff);
-    int status = -1;
-    if (w.iter >= max_iter) {
-        status = kTraceIterLimit;
-    } else if (w.ref == PICO_REF_DONE) {
-        status = kTraceOk;
-    } else {
-        ++w.iter;
-        if (!pico_is_leaf(w.ref)) {
-            float p[8], q[8];
-            load256(sc.nodes + w.ref, p);
-            load256(reinterpret_cast<const char*>(sc.nodes + w.ref) + 32, q);
-            const uint32_t ref0 = __float_as_uint(q[4]), ref1 = __float_as_uint(q[5]);
-            if (kCount) {
-                cnt->nodes++;
-                if (w.in_blas) cnt->blas_nodes++;
-            }
-            bool h0, h1;
-            float t0, t1;
-            if constexpr (kWT) {
-                t0 = slab_robust(p[0], p[2], p[1], p[3], q[0], q[1], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, w.cmag, h0);
-                t1 = slab_robust(p[4], p[6], p[5], p[7], q[2], q[3], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, w.cmag, h1);
-            } else if (w.cfast) {
-                const float2 nxy = make_float2(w.nx, w.ny), nzz = make_float2(w.nz, w.nz);
-                const float2 ixy = make_float2(w.cix, w.ciy), izz = make_float2(w.ciz, w.ciz);
-                t0 = slab_pairs(make_float2(p[0], p[1]), make_float2(p[2], p[3]), make_float2(q[0], q[1]), nxy, nzz,
-                                ixy, izz, h0);
-                t1 = slab_pairs(make_float2(p[4], p[5]), make_float2(p[6], p[7]), make_float2(q[2], q[3]), nxy, nzz,
-                                ixy, izz, h1);
-            } else {
-                t0 = slab(p[0], p[2], p[1], p[3], q[0], q[1], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, h0);
-                t1 = slab(p[4], p[6], p[5], p[7], q[2], q[3], -w.nx, -w.ny, -w.nz, w.cix, w.ciy, w.ciz, h1);
-            }
-            // t <= limit (finite) also rejects t = +inf and NaN, like "t <= best && t < inf"
-            const bool v0 = h0 && t0 <= w.limit;
-            const bool v1 = h1 && t1 <= w.limit;
-            if (v0 && v1) {
-                const bool swap = t1 < t0;
-                if (w.sp >= max_stack) {
-                    status = kTraceStackOverflow;
-                } else {
-                    stack[w.sp++] = swap ? ref0 : ref1;
-                    w.ref = swap ? ref1 : ref0;
-                }
-            } else if (v0) {
-                w.ref = ref0;
-            } else if (v1) {
-                w.ref = ref1;
-            } else {
-                w.ref = w.sp ? stack[--w.sp] : PICO_REF_DONE;
-            }
-        } else if (w.ref == PICO_REF_END_BLAS) {
-            // leave the instance: its candidate is the closest triangle by object-space t
-            if (w.ltri != kNoHit) {
-                const float tw = world_distance(sc, w.cur, w.ltri, w.lu, w.lv, w.o);
-                if (tw < w.best.t || (tw == w.best.t && w.cur < w.best.rank)) {
-                    w.best.t = tw; w.best.rank = w.cur; w.best.tri = w.ltri; w.best.u = w.lu; w.best.v = w.lv;
-                    if (tw < w.exit_below) status = kTraceOk;
-                }
-            }
-            w.in_blas = false;
-            // back to the world ray (its reciprocals recomputed rather than kept in registers)
-            w.nx = -w.o.x; w.ny = -w.o.y; w.nz = -w.o.z;
-            w.cix = __frcp_rn(w.d.x); w.ciy = __frcp_rn(w.d.y); w.ciz = __frcp_rn(w.d.z);
-            w.cfast = w.wfast;
-            w.cmag = w.wmag;
-            w.limit = fminf(w.best.t, kMaxFinite);
-            w.ref = w.sp ? stack[--w.sp] : PICO_REF_DONE;
-        } else {
-            const uint32_t first = pico_leaf_first(w.ref), count = pico_leaf_count(w.ref);
-            if (count == 0) {
-                w.ref = w.sp ? stack[--w.sp] : PICO_REF_DONE;
-            } else if (w.in_blas) {
-                for (uint32_t k = 0; k < count; ++k) {
-                    const uint32_t tri = first + k;
-                    float t, u, v;
-                    if (kCount) cnt->tris++;
-                    if (intersect<kWT>(sc.tris + tri, -w.nx, -w.ny, -w.nz, w.qdx, w.qdy, w.qdz, t, u, v) &&
-                        (t < w.lt || (t == w.lt && tri < w.ltri))) {
-                        w.lt = t; w.ltri = tri; w.lu = u; w.lv = v;
-                    }
-                }
-                w.limit = fminf(w.limit, w.lt);
-                w.ref = stack[--w.sp];   // the END_BLAS sentinel is below, so sp > 0 here
-            } else if (count > 1 && w.sp >= max_stack) {
-                status = kTraceStackOverflow;
-            } else {
-                // TLAS leaf: search the instance of item `first`; the rest of the leaf waits on the stack
-                if (count > 1) stack[w.sp++] = pico_leaf_ref(first + 1, count - 1);
-                const uint32_t rank = __ldg(sc.tlas_items + first);
-                if (kCount) cnt->insts++;
-                if (kImplicit && is_implicit_root(sc.insts + rank)) {
-                    // an implicit shape: one candidate, no BLAS and no root box test
-                    float tw, t;
-                    if (implicit_candidate(sc.insts + rank, w.o, w.d, tw, t) &&
-                        (tw < w.best.t || (tw == w.best.t && rank < w.best.rank))) {
-                        w.best.t = tw; w.best.rank = rank; w.best.tri = kImplicitTri; w.best.u = t; w.best.v = 0.0f;
-                        if (tw < w.exit_below) status = kTraceOk;
-                        w.limit = fminf(w.best.t, kMaxFinite);
-                    }
-                    w.ref = w.sp ? stack[--w.sp] : PICO_REF_DONE;
-                } else {
-                    const ObjectRay q = to_object(sc.insts + rank, w.o, w.d);
-                    // A triangle of an instance at object-space t lies at world distance t |D|
-                    // up to float error (relative ~1e-6, absolute ~1e-7 |O|); the BLAS bound
-                    // adds 0.1 % and 1e-4 (|O| + 1), far above that error, so it never cuts a
-                    // triangle that could beat or tie the best world distance.
-                    const float4 o = w.o, d = w.d;
-                    const float inv_len = rsqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
-                    const float omag = 1e-4f * (fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z)) + 1.0f);
-                    const float gl = (w.best.t * 1.001f + omag) * inv_len;
-                    bool h;
-                    const float qmag = kWT ? max_abs3(q.ox, q.oy, q.oz) : 0.0f;
-                    const float tm = box_test<kWT>(q.root_lo.x, q.root_hi.x, q.root_lo.y, q.root_hi.y, q.root_lo.z,
-                                                   q.root_hi.z, q.ox, q.oy, q.oz, q.ix, q.iy, q.iz, qmag, false, h);
-                    if (!(h && tm < kInf && tm <= gl)) {
-                        w.ref = w.sp ? stack[--w.sp] : PICO_REF_DONE;
-                    } else if (w.sp >= max_stack) {
-                        status = kTraceStackOverflow;
-                    } else {
-                        stack[w.sp++] = PICO_REF_END_BLAS;
-                        w.in_blas = true;
-                        w.nx = -q.ox; w.ny = -q.oy; w.nz = -q.oz; w.cix = q.ix; w.ciy = q.iy; w.ciz = q.iz;
-                        w.qdx = q.dx; w.qdy = q.dy; w.qdz = q.dz;
-                        w.cfast = sc.finite_boxes && all_finite(q.ox, q.oy, q.oz, q.ix, q.iy, q.iz);
-                        w.cmag = qmag;
-                        w.limit = fminf(gl, kMaxFinite);   // lt starts at +inf
-                        w.cur = rank;
-                        w.lt = kInf; w.ltri = kNoHit;
-                        w.ref = __float_as_uint(q.root_lo.w);
-                    }
-                }
-            }
+    ++w.iter;
+    const uint32_t first = pico_leaf_first(w.ref), count = pico_leaf_count(w.ref);
+    if (count == 0) {
+        nf_pop(w, mem);
+        return kWalking;
+    }
+    if (count > 1) {
+        if (w.sp >= max_stack) return kTraceStackOverflow;
+        mem[w.sp++] = pico_leaf_ref(first + 1, count - 1);
+    }
+    const uint32_t rank = tlas_rank(sc, first);
+    if (kCount) cnt->insts++;
+    const float4 o = nf_origin(mem);
+    const float4 d = make_float4(mem_float(mem, kMemD), mem_float(mem, kMemD + 1), mem_float(mem, kMemD + 2), 0.0f);
+    if (kImplicit && is_implicit_root(sc.insts + rank)) {
+        // an implicit shape: one candidate, no BLAS and no root box test
+        float tw, t;
+        int status = kWalking;
+        if (implicit_candidate(sc.insts + rank, o, d, tw, t)) {
+            if (nf_candidate(mem, tw, rank, kImplicitTri, t, 0.0f)) status = kTraceOk;
+            w.limit = fminf(mem_float(mem, kMemT), kMaxFinite);
         }
+        nf_pop(w, mem);
+        return status;
     }
-    return status;
-}
-
-// Whether a lane's next move waits: a move other than an inner node (a leaf, an
-// instance entry or exit, or handing in a finished walk) waits while lanes of the
-// warp walk inner nodes, until 5/8 of the busy lanes wait.  The warp then runs
-// those rarer branches for many lanes at once instead of for one or two in most
-// of its steps.  Measured on the 1080p lit-field renders, first with warps that
-// held their 32 rays to the end, against no waiting: a fixed count of 4 waiting
-// lanes 1.5 % slower, 8 2.4 % faster, 12 3.4 %, 16 2.8 %, 20 1.6 %, 24 no
-// faster, 32 (a while-while walk) 1.5 % slower; exempting the BLAS leaves 9 %
-// slower; a share of the busy lanes instead of a count: 3/8 6 %, 7/16 6.8 %,
-// 1/2 7.1 %, 9/16 6.6 %, 5/8 6.5 %, 3/4 5.1 % faster; releasing one kind of move
-// at a time 2 % slower than all at once.  Then with idle lanes refilled (see
-// walk_queue), against 1/2: 3/8 4.8 % slower, 5/8 1.3 % faster, 11/16 1.0 %,
-// 3/4 no faster, 7/8 2.5 % slower.  `busy`: the lanes holding a walk, `inner`:
-// this lane's next move is an inner node (false for a lane without a walk).
-// Every lane of `busy` must call it.
-__device__ __forceinline__ bool nf_release(unsigned busy, bool inner, unsigned& at_node)
-{
-    at_node = __ballot_sync(busy, inner);
-    return at_node == 0 || 8 * __popc(busy & ~at_node) >= 5 * __popc(busy);
-}
-
-// One ray's closest hit by the near-first walk (or its occlusion query, kAnyHit).
-template <bool kCount, bool kImplicit, bool kAnyHit = false, bool kRuntimeBounds = false, bool kWT = false>
-__device__ __forceinline__ int trace_near_first(const SceneView& sc, const float4 o, const float4 d, TraceHit& best,
-                                                TraceCounters* cnt, float tmax = INFINITY,
-                                                float exit_below = -INFINITY)
-{
-    NearFirstState w;
-    uint32_t stack[kTraceStack];
-    nf_start<kWT>(w, sc, o, d, tmax, exit_below, kAnyHit);
-    int status;
-    for (;;) {
-        // lanes that finished their walk have left the loop: the rest of the warp is busy
-        unsigned at_node;
-        const bool inner = !pico_is_leaf(w.ref);
-        if (!nf_release(__activemask(), inner, at_node) && !inner) continue;
-        status = nf_move<kCount, kImplicit, kRuntimeBounds, kWT>(w, sc, stack, cnt);
-        if (status >= 0) break;
+    const ObjectRay q = to_object(sc.insts + rank, o, d);
+    // A triangle of an instance at object-space t lies at world distance t |D|
+    // up to float error (relative ~1e-6, absolute ~1e-7 |O|); the BLAS bound
+    // adds 0.1 % and 1e-4 (|O| + 1), far above that error, so it never cuts a
+    // triangle that could beat or tie the best world distance.
+    const float inv_len = rsqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
+    const float omag = 1e-4f * (fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z)) + 1.0f);
+    const float gl = (mem_float(mem, kMemT) * 1.001f + omag) * inv_len;
+    const bool fast = sc.finite_boxes && all_finite(q.ox, q.oy, q.oz, q.ix, q.iy, q.iz);
+    bool h;
+    const float qmag = kWT ? max_abs3(q.ox, q.oy, q.oz) : 0.0f;
+    const float tm = box_test<kWT>(q.root_lo.x, q.root_hi.x, q.root_lo.y, q.root_hi.y, q.root_lo.z, q.root_hi.z, q.ox,
+                                   q.oy, q.oz, q.ix, q.iy, q.iz, qmag, fast, h);
+    if (!(h && tm < kInf && tm <= gl)) {
+        nf_pop(w, mem);
+        return kWalking;
     }
-    best = w.best;
-    if (kAnyHit && best.tri == kNoHit) best.rank = kNoHit;
-    return status;
+    if (w.sp >= max_stack) return kTraceStackOverflow;
+    mem[w.sp++] = PICO_REF_END_BLAS;
+    w.in_blas = true;
+    w.nx = -q.ox; w.ny = -q.oy; w.nz = -q.oz; w.cix = q.ix; w.ciy = q.iy; w.ciz = q.iz;
+    w.qdx = q.dx; w.qdy = q.dy; w.qdz = q.dz;
+    w.cfast = fast;
+    w.cmag = qmag;
+    w.limit = fminf(gl, kMaxFinite);   // lt starts at +inf
+    mem[kMemCur] = rank;
+    w.lt = kInf;
+    mem[kMemLtri] = kNoHit;
+    w.ref = __float_as_uint(q.root_lo.w);
+    return kWalking;
 }
 
-// Walks every ray of a queue of n entries with a warp's lanes, refilling idle
-// lanes in batches.  The walks and their hits are trace_near_first's; only the
-// order in which a warp's lanes make their moves differs.  `Rays` supplies the
+// The rarer moves of a walk that is not at an inner node, one after the other while the next one is of a later
+// kind: a BLAS leaf, then the exit it may pop, then the instance entry that may pop, then the walk's end.
+template <bool kCount, bool kImplicit, bool kRuntimeBounds, bool kWT>
+__device__ __forceinline__ int nf_rare(NearFirstState& w, const SceneView& sc, uint32_t* mem, TraceCounters* cnt)
+{
+    const uint32_t max_iter = kRuntimeBounds ? sc.max_iterations : kTraceMaxIter;
+    if (w.iter >= max_iter) return kTraceIterLimit;
+    if (w.in_blas && w.ref != PICO_REF_END_BLAS) {
+        nf_leaf<kCount, kWT>(w, sc, mem, cnt);
+        if (kRuntimeBounds && w.iter >= max_iter) return kTraceIterLimit;
+    }
+    if (w.ref == PICO_REF_END_BLAS) {
+        const int status = nf_exit(w, sc, mem);
+        if (status != kWalking) return status;
+        if (kRuntimeBounds && w.iter >= max_iter) return kTraceIterLimit;
+    }
+    if (!w.in_blas && pico_is_leaf(w.ref) && w.ref != PICO_REF_DONE) {
+        const int status = nf_enter<kCount, kImplicit, kRuntimeBounds, kWT>(w, sc, mem, cnt);
+        if (status != kWalking) return status;
+        if (kRuntimeBounds && w.iter >= max_iter) return kTraceIterLimit;
+    }
+    return w.ref == PICO_REF_DONE ? (int)kTraceOk : kWalking;
+}
+
+// Walks every ray of a queue of n entries with a warp's lanes.  `Rays` supplies the
 // entries:
 //   rays.load(k, o, d, tmax, exit_below, occlusion) -> a lane tag for entry k,
 //   rays.finish(tag, best, status) hands in a finished walk;
-// `Rays::Tag` is the tag's type, `Rays::Index` that of the entry indices.  A
-// lane whose walk ended waits (see
-// nf_release) to hand it in; once kRefillIdle lanes of the warp are idle they
-// take the next entries of the warp's claim together, and the warp claims
-// kClaim entries of the shared counter `work` at a time.  The earlier form, a
-// warp holding its 32 rays until the slowest ended, left lanes idle for most
-// of a walk's tail.  The 1080p renders: refilling at 8 idle lanes with one
-// atomic per refill 4.4 % faster (16 lanes 2.3 %, 12 4.3 %, 4 2.2 %, 2 and 1
-// slower), then claims of 64 entries another 4.8 % (the atomics on one counter
-// had become frequent), but 35 % slower Cornell-box renders, whose launches
-// hold a few dozen rays per warp: a warp then walked two or three claims'
-// worth of rays while others had none, so a launch with fewer than kClaim rays
-// per warp claims 32 at a time (the Cornell box back to 21 % slower than before
-// the refills, the 1080p renders unchanged), and the bar at 1024 rays per warp
-// instead of 64 brought the Cornell box to 17 % slower (the 1080p renders 0.1 %
-// faster); refilling only fully idle warps below the bar would bring it to 8 %
-// slower but cost the 1080p renders 1.5 %, whose small late-depth launches are
-// long-tailed.  A 32-bit Index for queues of fewer than 2^32 entries keeps the
-// extension kernel free of spills.
+// `Rays::Tag` is the tag's type, `Rays::Index` that of the entry indices.
+//
+// The walk is bound by instruction issue, and rays of one warp differ in where
+// they are, so the loop is built to run each branch for many lanes at once.  A
+// round moves the lanes at inner nodes (kInnerMoves moves each while they stay
+// there); the other lanes wait until kReleaseWait / 8 of the walking lanes wait, and
+// are then released through the rarer moves in the order a walk mostly meets them:
+// the leaf, the exit that leaf's pop may bring, the entry the exit's pop may bring
+// (nf_rare).  A walk that ended keeps its lane until kRefillIdle lanes are idle;
+// those hand in their results together and take the next entries of the warp's
+// claim together, and the warp claims kClaim entries of the shared counter `work`
+// at a time.  What only the rarer moves use is kept in local memory, so that nine
+// CTAs of 128 threads (56 registers) fit an SM without spills.
+//
+// Measured on the closest-hit benchmark (16.8M rays, half primary, half bounces) and
+// the 1080p lit-field render, identical hits and images: one rare move per release,
+// results handed in as one of them, all state in 64 registers 12.13 / 85.7 ms; the
+// rarer moves in a chain, results handed in at refills, their state in local memory
+// 11.43 / 80.6 ms; nine CTAs per SM instead of eight 10.90 / 77.6 ms (ten, with 50 to
+// 70 B of spills: 11.66 / 77.8); two inner moves per round 10.51 / 75.6 ms (three 10.62
+// / 76.1, four 10.76 / 76.8).  Around that: a wait of 4/8 instead of 5/8 no different,
+// 6/8 1.5 % slower; refilling at 4 idle lanes 1.8 % slower, at 12 no different; the
+// chain run twice or four times per release 1.7 to 3 % slower; a leaf's two triangles
+// tested at once in packed arithmetic (spills) 12 % slower.  Earlier forms: no waiting
+// 7 % slower than waiting, warps that held their 32 rays until the slowest ended another
+// 4.4 %, claims of 32 entries with one atomic per refill 4.8 %.
+//
+// A launch with fewer than kBigLaunch rays per warp claims 32 entries at a time, so that
+// its rays spread over the warps (the Cornell box at 256 x 256 has a few dozen rays per
+// warp and launch).  A 32-bit Index suffices for queues of fewer than 2^32 entries.
+constexpr int kReleaseWait = 5;   // of 8 walking lanes
+constexpr int kInnerMoves = 2;
 constexpr uint32_t kRefillIdle = 8;
 constexpr uint32_t kClaim = 64;   // queue entries a warp claims at a time
 // A claim must cover a refill of all 32 lanes, or the claimed range [next, end)
@@ -706,17 +761,24 @@ __device__ __forceinline__ void walk_queue(const SceneView& sc, Rays& rays, type
     using Index = typename Rays::Index;
     const unsigned lane = threadIdx.x & 31u;
     NearFirstState w;
-    uint32_t stack[kTraceStack];
+    uint32_t mem[kMemWords];
     typename Rays::Tag tag = 0;
-    bool live = false;
-    unsigned busy = 0;   // warp-uniform: the lanes holding a walk (lanes whose walk ended on a bound may linger)
+    int status = kIdle;
+    unsigned busy = 0;   // warp-uniform: the lanes that were walking at the last release
     bool more = true;    // warp-uniform: the queue may hold entries
     Index next = 0, end = 0;   // warp-uniform: the warp's claimed entries [next, end)
     // a launch with fewer than kBigLaunch rays per warp claims 32 at a time, so that its rays spread over the warps
     const bool big = (uint64_t)n >= (uint64_t)gridDim.x * (blockDim.x >> 5) * kBigLaunch;
     const uint32_t claim = big ? kClaim : 32u;
     for (;;) {
-        if (more && __popc(busy) <= 32 - kRefillIdle) {
+        if (more ? __popc(busy) <= 32 - kRefillIdle : busy == 0) {
+            if (status >= 0) {
+                const TraceHit best{mem_float(mem, kMemT), mem[kMemRank], mem[kMemTri], mem_float(mem, kMemU),
+                                    mem_float(mem, kMemV)};
+                rays.finish(tag, best, status);
+                status = kIdle;
+            }
+            if (!more) break;
             const unsigned idle = ~busy;
             const uint32_t need = __popc(idle);
             const uint32_t avail = (uint32_t)(end - next);
@@ -740,31 +802,32 @@ __device__ __forceinline__ void walk_queue(const SceneView& sc, Rays& rays, type
             } else {
                 next += need;
             }
-            if (!live && ((idle >> lane) & 1u) && k < n && (r < avail || more)) {
+            if (((idle >> lane) & 1u) && k < n && (r < avail || more)) {
                 float4 o, d;
                 float tmax, exit_below;
                 bool occlusion;
                 tag = rays.load(k, o, d, tmax, exit_below, occlusion);
-                nf_start<kWT>(w, sc, o, d, tmax, exit_below, occlusion);
-                live = true;
+                nf_start<kWT>(w, mem, sc, o, d, tmax, exit_below, occlusion);
+                status = kWalking;
             }
-            busy = __ballot_sync(0xffffffffu, live);
+            busy = __ballot_sync(0xffffffffu, status == kWalking);
+            if (busy == 0) continue;
         }
-        if (busy == 0) {
-            if (!more) break;
-            continue;
+        const bool inner = status == kWalking && !pico_is_leaf(w.ref);
+        const unsigned at_node = __ballot_sync(0xffffffffu, inner);
+        const bool release = at_node == 0 || 8 * __popc(busy & ~at_node) >= kReleaseWait * __popc(busy);
+        if (inner) {
+            status = nf_inner<kCount, kRuntimeBounds, kWT>(w, sc, mem, cnt);
+#pragma unroll
+            for (int k = 1; k < kInnerMoves; ++k)
+                if (status == kWalking && !pico_is_leaf(w.ref))
+                    status = nf_inner<kCount, kRuntimeBounds, kWT>(w, sc, mem, cnt);
         }
-        unsigned at_node;
-        const bool inner = live && !pico_is_leaf(w.ref);
-        const bool release = nf_release(0xffffffffu, inner, at_node);
-        if (live && (inner || release)) {
-            const int status = nf_move<kCount, kImplicit, kRuntimeBounds, kWT>(w, sc, stack, cnt);
-            if (status >= 0) {
-                rays.finish(tag, w.best, status);
-                live = false;
-            }
+        if (release) {
+            if (status == kWalking && pico_is_leaf(w.ref))
+                status = nf_rare<kCount, kImplicit, kRuntimeBounds, kWT>(w, sc, mem, cnt);
+            busy = __ballot_sync(0xffffffffu, status == kWalking);
         }
-        if (release) busy = __ballot_sync(0xffffffffu, live);
     }
 }
 
@@ -862,7 +925,7 @@ __device__ __forceinline__ int trace_reference_order(const SceneView& sc, const 
             if (sp >= max_stack) return kTraceStackOverflow;
             stack[sp++] = StackEntry{pico_leaf_ref(first + 1, count - 1), -kInf};
         }
-        const uint32_t rank = __ldg(sc.tlas_items + first);   // the identity on the reference's tree
+        const uint32_t rank = tlas_rank(sc, first);
         if (kCount) cnt->insts++;
         if (kImplicit && is_implicit_root(sc.insts + rank)) {
             float tw, t;
@@ -891,18 +954,14 @@ __device__ __forceinline__ int trace_reference_order(const SceneView& sc, const 
     return kTraceOk;
 }
 
-// The closest hit; the near-first walk may return early with a hit below
-// exit_below instead (see trace_near_first), the reference order never does.
+// The closest hit in the reference order.
 template <bool kCount, int kVariant>
 __device__ __forceinline__ int trace_closest(const SceneView& sc, const float4 o, const float4 d, TraceHit& best,
-                                             TraceCounters* cnt, float exit_below = -INFINITY)
+                                             TraceCounters* cnt)
 {
-    constexpr bool kImplicit = (kVariant & kWithImplicit) != 0;
-    constexpr bool kRuntime = (kVariant & kBounded) != 0;
-    constexpr bool kWT = (kVariant & kWatertight) != 0;
-    if ((kVariant & kReferenceOrder) != 0)
-        return trace_reference_order<kCount, kImplicit, kRuntime, kWT>(sc, o, d, best, cnt);
-    return trace_near_first<kCount, kImplicit, false, kRuntime, kWT>(sc, o, d, best, cnt, INFINITY, exit_below);
+    static_assert((kVariant & kReferenceOrder) != 0, "the near-first order walks queues (walk_queue)");
+    return trace_reference_order<kCount, (kVariant & kWithImplicit) != 0, (kVariant & kBounded) != 0,
+                                 (kVariant & kWatertight) != 0>(sc, o, d, best, cnt);
 }
 
 // A lower bound on the world distance of every hit on a NEE light seen from o:
@@ -926,25 +985,14 @@ __device__ __forceinline__ float light_distance_bound(const SceneView& sc, const
 }
 
 // Whether anything lies at a world distance below tmax along the ray (closest-hit
-// semantics: exactly when the closest hit is nearer than tmax).  The near-first
-// walk bounds its search by tmax and stops at the first such instance; the
-// reference order runs the closest hit.
-template <int kVariant, bool kCount = false>
+// semantics: exactly when the closest hit is nearer than tmax), in the reference order.
+template <int kVariant, bool kCount>
 __device__ __forceinline__ int trace_occluded(const SceneView& sc, const float4 o, const float4 d, float tmax,
-                                              bool& occluded, TraceCounters* cnt = nullptr)
+                                              bool& occluded, TraceCounters* cnt)
 {
-    constexpr bool kImplicit = (kVariant & kWithImplicit) != 0;
-    constexpr bool kRuntime = (kVariant & kBounded) != 0;
-    constexpr bool kWT = (kVariant & kWatertight) != 0;
     TraceHit h;
-    int s;
-    if ((kVariant & kReferenceOrder) != 0) {
-        s = trace_reference_order<kCount, kImplicit, kRuntime, kWT>(sc, o, d, h, cnt);
-        occluded = h.rank != kNoHit && h.t < tmax;
-    } else {
-        s = trace_near_first<kCount, kImplicit, true, kRuntime, kWT>(sc, o, d, h, cnt, tmax);
-        occluded = h.rank != kNoHit;
-    }
+    const int s = trace_closest<kCount, kVariant>(sc, o, d, h, cnt);
+    occluded = h.rank != kNoHit && h.t < tmax;
     return s;
 }
 
