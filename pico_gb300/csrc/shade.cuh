@@ -19,6 +19,7 @@
 #pragma once
 
 #include "exact_math.cuh"
+#include "float_pair.cuh"
 #include "kernels_render.h"
 #include "layout.h"
 #include "traverse.cuh"
@@ -141,11 +142,11 @@ __device__ __forceinline__ ex::V3 cos_sample(float u1, float u2)
 {
     using namespace ex;
     const float r = sqrt_(u1);
-    const float phi = (float)((double)u2 * kPi * 2.0);
+    const float phi = pair::two_pi_times(u2);
     const float om = sub(1.0f, u1);
-    const float z = (float)sqrt((double)((0.0f < om) ? om : 0.0f));
-    const double c = cos((double)phi), s = sin((double)phi);
-    return normalize(v3((float)((double)r * c), (float)((double)r * s), z));
+    const float z = sqrt_((0.0f < om) ? om : 0.0f);   // a double square root rounds to the same float
+    const float2 xy = pair::circle(r, phi);           // r cos(phi), r sin(phi) in double
+    return normalize(v3(xy.x, xy.y, z));
 }
 
 __device__ __forceinline__ float cos_pdf(ex::V3 H)
@@ -161,7 +162,7 @@ __device__ __forceinline__ ex::V3 beckmann_sample(float x0, float x1, ex::V3 V, 
     float log_sample = logf(sub(1.0f, x0));
     if (isinf(log_sample)) log_sample = 0.0f;
     const float tan2 = mul(mul(-alpha, alpha), log_sample);
-    const float phi = (float)((double)mul(x1, 2.0f) * kPi);
+    const float phi = pair::two_pi_times(x1);
     const float cos_t = div(1.0f, sqrt_(add(1.0f, tan2)));
     const float s2 = sub(1.0f, mul(cos_t, cos_t));
     const float sin_t = sqrt_((0.0f < s2) ? s2 : 0.0f);
@@ -196,7 +197,7 @@ __device__ __forceinline__ float beckmann_D(ex::V3 w, float R)
     const float sphi = (sin_t == 0.0f) ? 0.0f : clampf(div(w.y, sin_t), -1.0f, 1.0f);
     const float a2 = mul(ax, ax);
     const float e = expf(mul(-tan2, add(div(mul(cphi, cphi), a2), div(mul(sphi, sphi), a2))));
-    return (float)((double)e / (kPi * (double)ax * (double)ax * (double)cos4));
+    return pair::quotient_by_pi(e, ax, cos4);   // e / (pi ax^2 cos4) in double
 }
 
 __device__ __forceinline__ float beckmann_pdf(ex::V3 H, float R)
