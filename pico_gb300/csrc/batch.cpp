@@ -171,11 +171,11 @@ cudaError_t upload_render(const pico_render_item& it, BatchSlot& s, Prepared& pr
     active.clear();
     done.assign(pr.npx, 0u);
     pr.samples_before = 0;
-    for (size_t px = 0; px < pr.npx; ++px) {
+    for_tile_pixels(pr.W, pr.H, [&](uint32_t px) {
         pr.samples_before += it.sample_count[px];
         if (it.sample_count[px] >= cfg.max_samples) done[px] = 1;
-        else active.push_back((uint32_t)px);
-    }
+        else active.push_back(px);
+    });
     pr.nactive = active.size();
     pr.cam = make_camera_view(it.camera);
     cudaError_t e = r.pixels.reserve(pr.npx * 3 * sizeof(float));

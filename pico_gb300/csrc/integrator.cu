@@ -855,12 +855,13 @@ __global__ void __launch_bounds__(kRenderThreads) compact_pixels_kernel(RoundPla
 }
 
 // The image state of a render into caller buffers (pico_gpu_render_device).
-__global__ void __launch_bounds__(kRenderThreads) prepare_image_kernel(const uint32_t* count, uint32_t npx,
+__global__ void __launch_bounds__(kRenderThreads) prepare_image_kernel(const uint32_t* count, uint32_t W, uint32_t H,
                                                                       uint32_t max_samples, uint32_t* pix_list,
                                                                       uint32_t* done, uint32_t* taken)
 {
+    const uint32_t npx = W * H;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += gridDim.x * blockDim.x) {
-        pix_list[p] = p;
+        pix_list[p] = tile_pixel(p, W, H);
         done[p] = count[p] >= max_samples ? 1u : 0u;
         taken[p] = 0;
     }
@@ -872,7 +873,7 @@ struct GbufferRays {
     using Index = uint64_t;
     const SceneView& sc;
     const CameraView& cam;
-    uint32_t W;
+    uint32_t W, H;
     float* normals;
     float* positions;
     float* diffuse;
@@ -881,11 +882,12 @@ struct GbufferRays {
     __device__ __forceinline__ uint32_t load(uint64_t k, float4& o, float4& d, float& tmax, float& exit_below,
                                              bool& occlusion) const
     {
-        camera_ray(cam, 0.0f, 0.0f, (uint32_t)k % W, (uint32_t)k / W, o, d);
+        const uint32_t p = tile_pixel((uint32_t)k, W, H);
+        camera_ray(cam, 0.0f, 0.0f, p % W, p / W, o, d);
         tmax = INFINITY;
         exit_below = -INFINITY;
         occlusion = false;
-        return (uint32_t)k;
+        return p;
     }
 
     __device__ __forceinline__ void finish(uint32_t p, const TraceHit& h, int s) const
@@ -923,7 +925,7 @@ __global__ void __launch_bounds__(128) gbuffer_kernel(SceneView sc, CameraView c
                                                      float* normals, float* positions, float* diffuse,
                                                      unsigned long long* work, int* err)
 {
-    GbufferRays rays{sc, cam, W, normals, positions, diffuse, err};
+    GbufferRays rays{sc, cam, W, H, normals, positions, diffuse, err};
     const uint64_t npx = (uint64_t)W * H;
     if constexpr ((kOrder & kReferenceOrder) == 0) {
         TraceCounters cnt{0, 0, 0, 0};
@@ -1151,11 +1153,12 @@ cudaError_t launch_compact_pixels(RoundPlan* plan, const uint32_t* in, const uin
     return cudaGetLastError();
 }
 
-cudaError_t launch_prepare_image(const uint32_t* count, uint32_t npx, uint32_t max_samples, uint32_t* pix_list,
-                                 uint32_t* done, uint32_t* taken, cudaStream_t st)
+cudaError_t launch_prepare_image(const uint32_t* count, uint32_t W, uint32_t H, uint32_t max_samples,
+                                 uint32_t* pix_list, uint32_t* done, uint32_t* taken, cudaStream_t st)
 {
+    const uint32_t npx = W * H;
     if (npx == 0) return cudaSuccess;
-    prepare_image_kernel<<<grid_for(prepare_image_kernel, npx, kRenderThreads), kRenderThreads, 0, st>>>(count, npx, max_samples, pix_list,
+    prepare_image_kernel<<<grid_for(prepare_image_kernel, npx, kRenderThreads), kRenderThreads, 0, st>>>(count, W, H, max_samples, pix_list,
                                                                                   done, taken);
     return cudaGetLastError();
 }

@@ -418,11 +418,11 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
     if (host_list) {
         done.assign(npx, 0u);
         active.reserve(npx);
-        for (size_t p = 0; p < npx; ++p) {
+        for_tile_pixels(W, H, [&](uint32_t p) {
             samples_before += sample_count[p];
             if (sample_count[p] >= cfg->max_samples) done[p] = 1;
-            else active.push_back((uint32_t)p);
-        }
+            else active.push_back(p);
+        });
     }
     for (uint64_t& v : ctx->render_stats) v = 0;
     e = cudaMemcpyAsync(r.pixels.ptr, pixels, npx * 3 * sizeof(float), cudaMemcpyHostToDevice, st);
@@ -437,7 +437,7 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
                                 st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the host vectors end with this call
     } else if (e == cudaSuccess) {
-        e = launch_prepare_image(as<uint32_t>(r.count), (uint32_t)npx, cfg->max_samples, as<uint32_t>(r.pix_list),
+        e = launch_prepare_image(as<uint32_t>(r.count), W, H, cfg->max_samples, as<uint32_t>(r.pix_list),
                                  as<uint32_t>(r.done), as<uint32_t>(r.taken), st);
     }
     if (e != cudaSuccess) return cuda_error(ctx, e, "render upload");
@@ -498,7 +498,7 @@ int pico_gpu_render_device(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const
     for (DeviceBuffer* b : {&r.taken, &r.done, &r.pix_list})
         if (e == cudaSuccess) e = b->reserve(npx * sizeof(uint32_t));
     if (e != cudaSuccess) return cuda_error(ctx, e, "image state");
-    e = launch_prepare_image(d_count, (uint32_t)npx, cfg->max_samples, as<uint32_t>(r.pix_list), as<uint32_t>(r.done),
+    e = launch_prepare_image(d_count, cfg->width, cfg->height, cfg->max_samples, as<uint32_t>(r.pix_list), as<uint32_t>(r.done),
                              as<uint32_t>(r.taken), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->status->rays, 0, sizeof(ctx->status->rays), st);
     if (e != cudaSuccess) return cuda_error(ctx, e, "render set-up");

@@ -33,3 +33,24 @@ def test_denoiser_inputs_of_few_pixels(ctx, oracle, size):
     gs.free()
     for a, b in zip(got, want):
         np.testing.assert_array_equal(a, np.asarray(b).reshape(a.shape))
+
+
+@pytest.mark.parametrize("size", [(1, 1), (7, 9), (8, 8), (17, 5), (64, 31)])
+def test_tile_order_covers_ragged_images(ctx, size):
+    """Every pixel of images that do not divide into 8 x 8 tiles takes its samples once, on the device's list and
+    on the host-built one of batched renders, with the same result as when the whole image is one batch's chunk."""
+    gs = ctx.upload(scenes.cornell_box())
+    cam = scenes.cornell_camera(*size)
+    whole, count, _ = gs.render(cam, 4, 6, seed=3, estimator=1)
+    assert (count == 6).all()
+    try:
+        ctx.set_path_limit(64)
+        chunked, count, _ = gs.render(cam, 4, 6, seed=3, estimator=1)
+    finally:
+        ctx.set_path_limit(0)
+    items = [{"gpu_scene": gs, "camera": cam, "max_samples": 6, "max_depth": 4, "seed": 3, "estimator": 1}]
+    ctx.render_many(items)
+    gs.free()
+    assert (count == 6).all() and (items[0]["sample_count"] == 6).all()
+    np.testing.assert_array_equal(whole, chunked)
+    np.testing.assert_array_equal(whole, items[0]["pixels"])
