@@ -11,6 +11,8 @@ struct RenderBuffers {
     pico::DeviceBuffer pixels, variance, count, taken, done, pix_list;
     pico::DeviceBuffer pix_list2, plan;   // exit-aware rounds: the compacted pixel list, the round plan
     pico::DeviceBuffer gn, gp, gd, ga, gb, stats, out, tonemap;
+    pico::DeviceBuffer hdr_pix, hdr_codes, hdr_lens, hdr_off, hdr_body;   // .hdr output: image, codes, their lengths
+                                                                          // and places, the file's body
     // radiance cache: terminal queries / training records, record throughput and
     // payload, targets, previous roughness per path, entry counters
     pico::DeviceBuffer nrc_q, nrc_tp, nrc_tgt, nrc_prev, nrc_count;
@@ -20,7 +22,7 @@ struct RenderBuffers {
                                       &sorg, &sdir, &scontrib, &senergy, &q0, &q1, &sq, &counters, &pixels,
                                       &variance, &count, &taken, &done, &pix_list, &pix_list2, &plan, &gn, &gp, &gd,
                                       &ga, &gb, &stats,
-                                      &out, &tonemap, &nrc_q, &nrc_tp, &nrc_tgt, &nrc_prev, &nrc_count})
+                                      &out, &tonemap, &hdr_pix, &hdr_codes, &hdr_lens, &hdr_off, &hdr_body, &nrc_q, &nrc_tp, &nrc_tgt, &nrc_prev, &nrc_count})
             b->release();
     }
 };
