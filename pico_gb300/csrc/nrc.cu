@@ -8,12 +8,15 @@
 //
 // Both network kernels work on tiles of 128 queries, one per thread of a
 // warpgroup (4 warps), which is also one TMEM lane: the thread encodes its
-// query into row `tid` of a swizzled shared-memory tile, the group's first
+// query, eight inputs at a time, into row `tid` of a swizzled shared-memory tile, the group's first
 // thread issues the layer's tcgen05.mma (M = 128, N = 64 or 16, K = 64 as four
 // K = 16 steps) with the accumulator in TMEM and commits it to an mbarrier, and
 // every thread reads its row back with tcgen05.ld, applies ReLU and writes the
 // next layer's input tile.  Inference CTAs hold 1, 2 or 4 such groups on their
-// own tiles and TMEM columns; training CTAs hold one.  The weights (43 KB,
+// own tiles and TMEM columns (one CTA per SM: what their tiles leave of the L1 holds
+// the coarse grid levels, and a second CTA's tiles in its place took 1M queries from 253
+// to 505 us, as did 64 registers with two threads a row, to 293); in training four groups
+// share one tile, a quarter of the levels and columns each.  The weights (43 KB,
 // bf16, already in the swizzled layout) reach shared memory once per CTA with
 // one bulk copy.
 //
@@ -38,7 +41,6 @@ namespace nrc {
 
 namespace {
 
-constexpr int kThreads = 128;
 // Inference CTAs hold G warpgroups (128-row tiles in flight), G = 1, 2 or 4.
 constexpr uint32_t infer_smem(int G) { return kWeightRegion + (uint32_t)G * kTileBytes + 64 + 1024; }
 constexpr uint32_t infer_tmem_cols(int G) { return 64u * (uint32_t)G; }   // a power of two for G = 1, 2, 4
@@ -73,11 +75,16 @@ __global__ void __launch_bounds__(256) encode_kernel(GridGeometry g, const __hal
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const Query q = load_query(queries + 4 * (size_t)i);
-        float in[kWidth];
-        encode(g, table, q, in);
+        float u[3];
+        normalise_position(g, q, u);
         float4* o = reinterpret_cast<float4*>(out + (size_t)kWidth * i);
 #pragma unroll
-        for (int k = 0; k < kWidth / 4; ++k) o[k] = make_float4(in[4 * k], in[4 * k + 1], in[4 * k + 2], in[4 * k + 3]);
+        for (int c = 0; c < 8; ++c) {
+            float in[8];
+            encode_chunk(g, table, q, u, c, in);
+            o[2 * c] = make_float4(in[0], in[1], in[2], in[3]);
+            o[2 * c + 1] = make_float4(in[4], in[5], in[6], in[7]);
+        }
     }
 }
 
@@ -126,7 +133,7 @@ __device__ __forceinline__ bool group_sync_and(uint32_t g, bool v)
 }
 
 template <int G>
-__global__ void __launch_bounds__(128 * G) infer_kernel(InferArgs a)
+__global__ void __launch_bounds__(128 * G, 4 / G) infer_kernel(InferArgs a)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
@@ -164,16 +171,17 @@ __global__ void __launch_bounds__(128 * G) infer_kernel(InferArgs a)
         const bool valid = row < n;
         uint32_t payload = 0;
         {
-            float in[kWidth];
-            if (valid) {
-                const Query q = load_query(a.queries + 4 * (size_t)row);
-                payload = q.pad;
-                encode(a.g, a.table, q, in);
-            } else {
+            Query q{};
+            float u[3];
+            if (valid) q = load_query(a.queries + 4 * (size_t)row);
+            payload = q.pad;
+            normalise_position(a.g, q, u);
 #pragma unroll
-                for (int k = 0; k < kWidth; ++k) in[k] = 0.0f;
+            for (int c = 0; c < 8; ++c) {
+                float in[8] = {};
+                if (valid) encode_chunk(a.g, a.table, q, u, c, in);
+                store_chunk<false>(X, gtid, c, in);
             }
-            store_row<false>(X, gtid, in);
         }
         bool abort = false;
 #pragma unroll 1
@@ -190,10 +198,13 @@ __global__ void __launch_bounds__(128 * G) infer_kernel(InferArgs a)
             phase ^= 1u;
             tc_fence_after();
             if (l < kHidden) {
-                float v[kWidth];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) tmem_ld16(lane_addr + 16 * c, v + 16 * c);
-                store_row<true>(X, gtid, v);
+                for (int c = 0; c < 4; ++c) {
+                    float v[16];
+                    tmem_ld16(lane_addr + 16 * c, v);
+                    store_chunk<true>(X, gtid, 2 * c, v);
+                    store_chunk<true>(X, gtid, 2 * c + 1, v + 8);
+                }
             } else {
                 float v[16];
                 tmem_ld16(lane_addr, v);
@@ -228,13 +239,19 @@ struct TrainArgs {
     TrainBatch b;
     float loss_scale;      // 1 / (3 n)
     float2* grid_grad;
+    float2* replicas;      // kReplicas copies of the replicated levels' gradients, or null
     float* partial;        // [gridDim.x][kMlpParams]
     float* loss;
     int* err;
     WaitPolicy wait;
 };
 
-__global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
+// One 128-row tile at a time per CTA, shared by kTrainGroups warpgroups: four threads of different groups hold one
+// row (one TMEM lane).  Group w encodes levels 4 w to 4 w + 3 (and one of the other input chunks), reads columns 16 w to
+// 16 w + 15 of the accumulators back, and scatters its levels' gradients.
+constexpr int kTrainGroups = 4, kTrainThreads = 128 * kTrainGroups;
+
+__global__ void __launch_bounds__(kTrainThreads, 1) train_kernel(TrainArgs a)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = align1024(smem_raw);
@@ -243,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
     uint8_t* dY = X + 6 * kTileBytes;          // gradient at the current layer's output
     uint64_t* bars = reinterpret_cast<uint64_t*>(dY + kTileBytes + kGuardBytes);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, group = tid >> 7, r = tid & 127u;
     const uint32_t bar_w = smem_addr(bars), bar_m = smem_addr(bars + 1);
     if (tid == 0) {
         mbar_init(bar_w, 1);
@@ -264,19 +281,19 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
     }
     bool ok = mbar_wait(bar_w, 0, a.wait.limit_ns);
     uint32_t phase = 0;
-    const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
+    const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);
     const uint32_t w_addr = smem_addr(W), x_addr = smem_addr(X), dy_addr = smem_addr(dY);
     const uint32_t ntiles = (a.b.n + kRows - 1) / kRows;
     bool first = true;
     float loss_sum = 0.0f;
     bool abort = false;
     for (uint32_t t = blockIdx.x; t < ntiles && !abort; t += gridDim.x) {
-        const uint32_t row = t * kRows + tid;
+        const uint32_t row = t * kRows + r;
         bool valid = row < a.b.n;
         float u[3] = {0.0f, 0.0f, 0.0f};
         float target[3] = {0.0f, 0.0f, 0.0f};
         {
-            float in[kWidth];
+            float in[8] = {}, other[8] = {};
             if (valid) {
                 const size_t rec = a.b.offset + (size_t)row * a.b.stride;
                 const Query q = load_query(a.b.queries + 4 * rec);
@@ -284,12 +301,13 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
                 target[0] = tg.x; target[1] = tg.y; target[2] = tg.z;
                 valid = isfinite(tg.x) && isfinite(tg.y) && isfinite(tg.z);
                 normalise_position(a.g, q, u);
-                encode(a.g, a.table, q, in);
-            } else {
 #pragma unroll
-                for (int k = 0; k < kWidth; ++k) in[k] = 0.0f;
+                for (int k = 0; k < 4; ++k)
+                    grid_features(a.g, a.table, (int)(4 * group) + k, u, in[2 * k], in[2 * k + 1]);
+                encode_chunk(a.g, a.table, q, u, (int)(4 + group), other);
             }
-            store_row<false>(X, tid, in);
+            store_chunk<false>(X, r, group, in);
+            store_chunk<false>(X, r, 4 + group, other);
         }
         // forward
 #pragma unroll 1
@@ -305,26 +323,27 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
             ok = mbar_wait(bar_m, phase, a.wait.limit_ns);
             phase ^= 1u;
             tc_fence_after();
+            float v[16] = {};
             if (l < kHidden) {
-                float v[kWidth];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) tmem_ld16(lane_addr + 16 * c, v + 16 * c);
-                store_row<true>(X + (l + 1) * kTileBytes, tid, v);
+                tmem_ld16(lane_addr + 16 * group, v);
+                store_chunk<true>(X + (l + 1) * kTileBytes, r, 2 * group, v);
+                store_chunk<true>(X + (l + 1) * kTileBytes, r, 2 * group + 1, v + 8);
             } else {
-                float v[16];
-                tmem_ld16(lane_addr, v);
-                float d[kWidth];
+                // group 0 turns the outputs into the loss gradient; the other columns of dY are zero
+                float d[16] = {};
+                if (group == 0) {
+                    tmem_ld16(lane_addr, v);
+                    if (valid) {
 #pragma unroll
-                for (int k = 0; k < kWidth; ++k) d[k] = 0.0f;
-                if (valid) {
-#pragma unroll
-                    for (int c = 0; c < kOutputs; ++c) {
-                        const float y = v[c], den = y * y + 0.01f, diff = y - target[c];
-                        loss_sum += diff * diff / den * a.loss_scale;
-                        d[c] = 2.0f * diff / den * a.loss_scale;
+                        for (int c = 0; c < kOutputs; ++c) {
+                            const float y = v[c], den = y * y + 0.01f, diff = y - target[c];
+                            loss_sum += diff * diff / den * a.loss_scale;
+                            d[c] = 2.0f * diff / den * a.loss_scale;
+                        }
                     }
                 }
-                store_row<false>(dY, tid, d);
+                store_chunk<false>(dY, r, 2 * group, d);
+                store_chunk<false>(dY, r, 2 * group + 1, d + 8);
             }
         }
         if (abort) break;
@@ -350,14 +369,13 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
             ok = mbar_wait(bar_m, phase, a.wait.limit_ns);
             phase ^= 1u;
             tc_fence_after();
-            float v[kWidth];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) tmem_ld16(lane_addr + 16 * c, v + 16 * c);
             if (l > 0) {
+                float v[16];
+                tmem_ld16(lane_addr + 16 * group, v);
                 const uint8_t* xl = X + l * kTileBytes;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 w = *reinterpret_cast<const uint4*>(xl + swz(tid, c));
+                for (int c = 0; c < 2; ++c) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(xl + swz(r, 2 * group + c));
                     const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
@@ -365,23 +383,30 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
                         if ((ws[k] & 0x8000u) || !(ws[k] & 0x7fffu)) v[8 * c + 2 * k] = 0.0f;
                         if ((ws[k] & 0x80000000u) || !(ws[k] & 0x7fff0000u)) v[8 * c + 2 * k + 1] = 0.0f;
                     }
+                    store_chunk<false>(dY, r, 2 * group + c, v + 8 * c);
                 }
-                store_row<false>(dY, tid, v);
-            } else if (valid) {
-#pragma unroll 1
-                for (int lev = 0; lev < kLevels; ++lev) {
-                    uint32_t c[3];
-                    float f[3];
-                    grid_cell(a.g, lev, u, c, f);
-                    const float g0 = v[kInputHash + 2 * lev], g1 = v[kInputHash + 2 * lev + 1];
-                    float2* lv = a.grid_grad + ((size_t)lev << a.g.log2_table);
+            } else {
+                float v[8];   // the gradients of the group's four levels' features
+                tmem_ld8(lane_addr + kInputHash + 8 * group, v);
+                if (valid) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const uint32_t dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
-                        const float w = (dx ? f[0] : 1.0f - f[0]) * (dy ? f[1] : 1.0f - f[1]) *
-                                        (dz ? f[2] : 1.0f - f[2]);
-                        atomicAdd(lv + grid_index(a.g, lev, c[0] + dx, c[1] + dy, c[2] + dz),
-                                  make_float2(w * g0, w * g1));
+                    for (int k = 0; k < 4; ++k) {
+                        const int lev = (int)(4 * group) + k;
+                        uint32_t c[3];
+                        float f[3];
+                        grid_cell(a.g, lev, u, c, f);
+                        const float g0 = v[2 * k], g1 = v[2 * k + 1];
+                        float2* lv = a.grid_grad + ((size_t)lev << a.g.log2_table);
+                        if (a.replicas && a.g.rep_base[lev] != kNoReplica)
+                            lv = a.replicas + (size_t)(blockIdx.x % kReplicas) * a.g.rep_entries + a.g.rep_base[lev];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const uint32_t dx = e & 1, dy = (e >> 1) & 1, dz = e >> 2;
+                            const float w = (dx ? f[0] : 1.0f - f[0]) * (dy ? f[1] : 1.0f - f[1]) *
+                                            (dz ? f[2] : 1.0f - f[2]);
+                            atomicAdd(lv + grid_index(a.g, lev, c[0] + dx, c[1] + dy, c[2] + dz),
+                                      make_float2(w * g0, w * g1));
+                        }
                     }
                 }
             }
@@ -389,17 +414,19 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
         first = false;
     }
     // loss of the CTA
-    for (int o = 16; o > 0; o >>= 1) loss_sum += __shfl_xor_sync(0xffffffffu, loss_sum, o);
-    if (lane == 0 && loss_sum != 0.0f) atomicAdd(a.loss, loss_sum);
-    // the CTA's weight-gradient partial: TMEM lanes = output rows
+    if (group == 0) {
+        for (int o = 16; o > 0; o >>= 1) loss_sum += __shfl_xor_sync(0xffffffffu, loss_sum, o);
+        if (lane == 0 && loss_sum != 0.0f) atomicAdd(a.loss, loss_sum);
+    }
+    // the CTA's weight-gradient partial: TMEM lanes = output rows, the layers shared out over the groups
     tc_fence_before();
     const bool good = __syncthreads_and(ok && !abort);   // block-uniform: tcgen05.ld needs whole warps
     tc_fence_after();
-    if (good && warp < 2) {
+    if (good && (warp & 3u) < 2) {
         float* part = a.partial + (size_t)blockIdx.x * kMlpParams;
-        const uint32_t o = warp * 32u + lane;
-        for (int l = 0; l < kLayers; ++l) {
-            if (l == kHidden && warp > 0) break;   // the output layer has 16 rows
+        const uint32_t o = (warp & 3u) * 32u + lane;
+        for (int l = (int)group; l < kLayers; l += kTrainGroups) {
+            if (l == kHidden && (warp & 3u) > 0) break;   // the output layer has 16 rows
             float* dst = part + (size_t)l * kWidth * kWidth + (size_t)o * kWidth;
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
@@ -418,16 +445,45 @@ __global__ void __launch_bounds__(kThreads, 1) train_kernel(TrainArgs a)
 }
 
 // ------------------------------------------------------------------ optimiser
-__global__ void __launch_bounds__(256) adam_mlp_kernel(const float* __restrict__ partial, uint32_t parts,
-                                                      float* master, float* m, float* v, float* grad, uint8_t* image,
-                                                      AdamStep s, bool apply)
+// The gradients a training step left in pieces: the weights' per-CTA partials, eight threads a weight and summed in
+// a fixed order, with the weights' optimiser step (blocks below kMlpBlocks), and the replicated grid levels' copies
+// (the blocks above).  One thread a weight over all partials took 10.5 us, this 4.
+constexpr uint32_t kMlpBlocks = kMlpParams / 32;
+static_assert(kMlpParams % 32 == 0, "whole warps of weights");
+
+__global__ void __launch_bounds__(256) gather_gradients_kernel(GridGeometry geo, const float* __restrict__ partial,
+                                                              uint32_t parts, float* master, float* m, float* v,
+                                                              float* grad, uint8_t* image, AdamStep s, bool apply,
+                                                              const float2* __restrict__ replicas, float2* grid_grad)
 {
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= kMlpParams) return;
+    if (blockIdx.x >= kMlpBlocks) {
+        const uint32_t e = (blockIdx.x - kMlpBlocks) * 256 + threadIdx.x;
+        if (e >= geo.rep_entries) return;
+        float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < kReplicas; ++k) {
+            const float2 r = replicas[(size_t)k * geo.rep_entries + e];
+            sum.x += r.x;
+            sum.y += r.y;
+        }
+        int lev = 0;
+        for (int l = 0; l < kLevels; ++l)
+            if (geo.rep_base[l] != kNoReplica && geo.rep_base[l] <= e) lev = l;   // the bases ascend
+        grid_grad[((size_t)lev << geo.log2_table) + (e - geo.rep_base[lev])] = sum;
+        return;
+    }
+    __shared__ float slice[8][32];
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, idx = blockIdx.x * 32 + lane;
+    float g = 0.0f;
+    for (uint32_t c = w; c < parts; c += 8) g += partial[(size_t)c * kMlpParams + idx];
+    slice[w][lane] = g;
+    __syncthreads();
+    if (w > 0) return;
+    g = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) g += slice[k][lane];
     const uint32_t l = idx / (kWidth * kWidth), o = (idx / kWidth) % kWidth, i = idx % kWidth;
     if (l == kHidden && o >= (uint32_t)kOutputs) return;   // padding rows stay zero
-    float g = 0.0f;
-    for (uint32_t c = 0; c < parts; ++c) g += partial[(size_t)c * kMlpParams + idx];
     grad[idx] = g;
     if (!apply) return;
     const float mm = s.beta1 * m[idx] + (1.0f - s.beta1) * g;
@@ -542,7 +598,7 @@ cudaError_t launch_infer(const GridGeometry& g, const __half2* table, const uint
 }
 
 cudaError_t launch_train(const GridGeometry& g, const __half2* table, const uint8_t* weights, const TrainBatch& b,
-                         float2* grid_grad, float* partial, uint32_t max_parts, uint32_t* parts, float* loss,
+                         float2* grid_grad, float2* replicas, float* partial, uint32_t max_parts, uint32_t* parts, float* loss,
                          int* err, cudaStream_t st, const WaitPolicy& wait)
 {
     *parts = 0;
@@ -555,16 +611,19 @@ cudaError_t launch_train(const GridGeometry& g, const __half2* table, const uint
     }
     uint32_t grid = train_grid_size(b.n);
     if (grid > max_parts) grid = max_parts;
-    TrainArgs a{g, table, weights, b, 1.0f / (3.0f * (float)b.n), grid_grad, partial, loss, err, wait};
-    train_kernel<<<grid, kThreads, kTrainSmem, st>>>(a);
+    TrainArgs a{g, table, weights, b, 1.0f / (3.0f * (float)b.n), grid_grad, replicas, partial, loss, err, wait};
+    train_kernel<<<grid, kTrainThreads, kTrainSmem, st>>>(a);
     *parts = grid;
     return cudaGetLastError();
 }
 
-cudaError_t launch_adam_mlp(const float* partial, uint32_t parts, float* master, float* m, float* v, float* grad,
-                            uint8_t* image, const AdamStep& s, bool apply, cudaStream_t st)
+cudaError_t launch_gather_gradients(const GridGeometry& g, const float* partial, uint32_t parts, float* master, float* m,
+                                    float* v, float* grad, uint8_t* image, const AdamStep& s, bool apply,
+                                    const float2* replicas, float2* grid_grad, cudaStream_t st)
 {
-    adam_mlp_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(partial, parts, master, m, v, grad, image, s, apply);
+    const uint32_t blocks = kMlpBlocks + (replicas ? (g.rep_entries + 255) / 256 : 0u);
+    gather_gradients_kernel<<<blocks, 256, 0, st>>>(g, partial, parts, master, m, v, grad, image, s, apply, replicas,
+                                                    grid_grad);
     return cudaGetLastError();
 }
 

@@ -46,15 +46,17 @@ cudaError_t launch_infer(const GridGeometry& g, const __half2* table, const uint
                          const uint32_t* n_dev = nullptr, int groups = 4, const WaitPolicy& wait = WaitPolicy{});
 // Gradients of the relative L2 loss over one batch: per-CTA weight-gradient
 // partials (kMlpParams floats each, returned count in *parts) and the hash-grid
-// gradient (accumulated into grid_grad, which the caller zeroes); adds the mean
-// loss to *loss.
+// gradient (accumulated into grid_grad and, with replicas, its replicated levels into
+// those copies instead; the caller zeroes both); adds the mean loss to *loss.
 cudaError_t launch_train(const GridGeometry& g, const __half2* table, const uint8_t* weights, const TrainBatch& b,
-                         float2* grid_grad, float* partial, uint32_t max_parts, uint32_t* parts, float* loss,
+                         float2* grid_grad, float2* replicas, float* partial, uint32_t max_parts, uint32_t* parts,
+                         float* loss,
                          int* err, cudaStream_t st, const WaitPolicy& wait = WaitPolicy{});
-// Sums the partials into grad; with apply, one Adam step on the master weights,
-// which are then written as the swizzled bf16 image.
-cudaError_t launch_adam_mlp(const float* partial, uint32_t parts, float* master, float* m, float* v, float* grad,
-                            uint8_t* image, const AdamStep& s, bool apply, cudaStream_t st);
+// Sums the partials into grad and the replicas into grid_grad; with apply, one Adam step
+// on the master weights, which are then written as the swizzled bf16 image.
+cudaError_t launch_gather_gradients(const GridGeometry& g, const float* partial, uint32_t parts, float* master, float* m,
+                                    float* v, float* grad, uint8_t* image, const AdamStep& s, bool apply,
+                                    const float2* replicas, float2* grid_grad, cudaStream_t st);
 cudaError_t launch_adam_grid(const float* grad, float* master, float* m, float* v, __half2* table, size_t nfloats,
                              const AdamStep& s, cudaStream_t st);
 cudaError_t launch_write_image(const float* master, uint8_t* image, cudaStream_t st);

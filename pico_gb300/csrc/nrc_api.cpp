@@ -65,6 +65,13 @@ void set_geometry(pico_gpu_nrc* c, const float lo[3], const float hi[3])
         const uint64_t r1 = (uint64_t)std::floor(s) + 2;
         g.res1[l] = (r1 * r1 * r1 <= T) ? (uint32_t)r1 : 0u;
     }
+    g.rep_entries = 0;
+    for (int l = 0; l < kLevels; ++l) {
+        const uint64_t r = g.res1[l], n = r * r * r;
+        const bool copied = r && n <= kReplicaMax;
+        g.rep_base[l] = copied ? g.rep_entries : kNoReplica;
+        if (copied) g.rep_entries += (uint32_t)n;
+    }
     g.table_mask = T - 1;
     g.log2_table = cfg.log2_table_size;
     for (int a = 0; a < 3; ++a) {
@@ -93,15 +100,24 @@ AdamStep next_adam_step(pico_gpu_nrc* c)
 int train_step(pico_gpu_nrc* c, const TrainBatch& b, bool apply, cudaStream_t st)
 {
     pico_gpu_ctx* ctx = c->ctx;
-    cudaError_t e = cudaMemsetAsync(c->grid_grad, 0, c->grid_floats * sizeof(float), st);
+    // the replicas lie behind the gradient, in one allocation
+    const bool copies = b.n >= kReplicaRecords && c->geo.rep_entries > 0;
+    float2* grid_grad = reinterpret_cast<float2*>(c->grid_grad);
+    float2* replicas = copies ? reinterpret_cast<float2*>(c->grid_grad + c->grid_floats) : nullptr;
+    cudaError_t e = cudaMemsetAsync(c->grid_grad, 0,
+                                    c->grid_floats * sizeof(float) +
+                                        (copies ? (size_t)kReplicas * c->geo.rep_entries * sizeof(float2) : 0),
+                                    st);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->loss, 0, sizeof(float), st);
     uint32_t parts = 0;
     if (e == cudaSuccess)
-        e = launch_train(c->geo, c->table, c->image, b, reinterpret_cast<float2*>(c->grid_grad), c->partial,
+        e = launch_train(c->geo, c->table, c->image, b, grid_grad, replicas, c->partial,
                          c->max_parts, &parts, c->loss, c->err, st, c->wait);
     if (e != cudaSuccess) return cuda_error(ctx, e, "radiance cache training");
     const AdamStep s = apply ? next_adam_step(c) : AdamStep{};
-    if (parts > 0) e = launch_adam_mlp(c->partial, parts, c->master, c->adam_m, c->adam_v, c->grad, c->image, s, apply, st);
+    if (parts > 0)
+        e = launch_gather_gradients(c->geo, c->partial, parts, c->master, c->adam_m, c->adam_v, c->grad, c->image, s,
+                                    apply, replicas, grid_grad, st);
     else e = cudaMemsetAsync(c->grad, 0, kMlpParams * sizeof(float), st);
     if (e == cudaSuccess && apply)
         e = launch_adam_grid(c->grid_grad, c->grid_master, c->grid_m, c->grid_v, c->table, c->grid_floats, s, st);
@@ -176,7 +192,7 @@ int pico_gpu_nrc_create(pico_gpu_ctx* ctx, const pico_nrc_config* cfg, pico_gpu_
     alloc(c->grid_master, c->grid_floats * sizeof(float));
     alloc(c->grid_m, c->grid_floats * sizeof(float));
     alloc(c->grid_v, c->grid_floats * sizeof(float));
-    alloc(c->grid_grad, c->grid_floats * sizeof(float));
+    alloc(c->grid_grad, c->grid_floats * sizeof(float) + (size_t)kReplicas * c->geo.rep_entries * sizeof(float2));
     alloc(c->table, c->grid_floats * sizeof(__half));
     alloc(c->loss, sizeof(float));
     alloc(c->err, sizeof(int));

@@ -78,39 +78,50 @@ __device__ __forceinline__ void sh16(float x, float y, float z, float* o)
     o[15] = -0.59004358992664352f * x * (xx - 3.0f * yy);
 }
 
-// The 64 network inputs of a query: 16 levels x 2 trilinearly interpolated
-// hash-grid features, 16 SH values of the direction, normal, roughness,
-// albedo, a constant 1 (the first layer's bias) and zero padding.
-__device__ __forceinline__ void encode(const GridGeometry& g, const __half2* __restrict__ table, const Query& q,
-                                       float* in)
+// One level's two features at a normalised point: trilinear interpolation over the cell's eight table entries.
+__device__ __forceinline__ void grid_features(const GridGeometry& g, const __half2* __restrict__ table, int l,
+                                              const float u[3], float& a0, float& a1)
 {
-    float u[3];
-    normalise_position(g, q, u);
+    uint32_t c[3];
+    float f[3];
+    grid_cell(g, l, u, c, f);
+    const __half2* lv = table + ((size_t)l << g.log2_table);
+    a0 = 0.0f;
+    a1 = 0.0f;
 #pragma unroll
-    for (int l = 0; l < kLevels; ++l) {
-        uint32_t c[3];
-        float f[3];
-        grid_cell(g, l, u, c, f);
-        const __half2* lv = table + ((size_t)l << g.log2_table);
-        float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
-            const float w = (dx ? f[0] : 1.0f - f[0]) * (dy ? f[1] : 1.0f - f[1]) * (dz ? f[2] : 1.0f - f[2]);
-            const float2 v = __half22float2(lv[grid_index(g, l, c[0] + dx, c[1] + dy, c[2] + dz)]);
-            a0 += w * v.x;
-            a1 += w * v.y;
-        }
-        in[kInputHash + 2 * l] = a0;
-        in[kInputHash + 2 * l + 1] = a1;
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
+        const float w = (dx ? f[0] : 1.0f - f[0]) * (dy ? f[1] : 1.0f - f[1]) * (dz ? f[2] : 1.0f - f[2]);
+        const float2 v = __half22float2(lv[grid_index(g, l, c[0] + dx, c[1] + dy, c[2] + dz)]);
+        a0 += w * v.x;
+        a1 += w * v.y;
     }
-    sh16(q.dx, q.dy, q.dz, in + kInputSH);
-    in[kInputNormal] = q.nx; in[kInputNormal + 1] = q.ny; in[kInputNormal + 2] = q.nz;
-    in[kInputRough] = q.rough;
-    in[kInputAlbedo] = q.ax; in[kInputAlbedo + 1] = q.ay; in[kInputAlbedo + 2] = q.az;
-    in[kInputBias] = 1.0f;
+}
+
+// The 64 network inputs of a query, eight at a time (chunk 0 to 7): 16 levels x 2 trilinearly interpolated hash-grid
+// features, 16 SH values of the direction, then normal, roughness, albedo and a constant 1 (the first layer's bias),
+// and zero padding.
+__device__ __forceinline__ void encode_chunk(const GridGeometry& g, const __half2* __restrict__ table, const Query& q,
+                                             const float u[3], int chunk, float (&in)[8])
+{
+    static_assert(kInputHash == 0 && kInputSH == 32 && kInputNormal == 48 && kInputRough == 51 && kInputAlbedo == 52 &&
+                      kInputBias == 55,
+                  "the chunks below hold these inputs");
+    if (chunk < 4) {
 #pragma unroll
-    for (int k = kInputBias + 1; k < kWidth; ++k) in[k] = 0.0f;
+        for (int k = 0; k < 4; ++k) grid_features(g, table, 4 * chunk + k, u, in[2 * k], in[2 * k + 1]);
+    } else if (chunk < 6) {
+        float sh[16];
+        sh16(q.dx, q.dy, q.dz, sh);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) in[k] = chunk == 4 ? sh[k] : sh[8 + k];
+    } else {
+        const bool last = chunk == 7;
+        in[0] = last ? 0.0f : q.nx; in[1] = last ? 0.0f : q.ny; in[2] = last ? 0.0f : q.nz;
+        in[3] = last ? 0.0f : q.rough;
+        in[4] = last ? 0.0f : q.ax; in[5] = last ? 0.0f : q.ay; in[6] = last ? 0.0f : q.az;
+        in[7] = last ? 0.0f : 1.0f;
+    }
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b)
@@ -119,20 +130,17 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b)
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Writes 64 floats as one bf16 row of a swizzled tile (relu: negative values to 0).
+// Writes eight floats as bf16 chunk `chunk` of a row of a swizzled tile (relu: negative values to 0).
 template <bool kRelu>
-__device__ __forceinline__ void store_row(uint8_t* tile, uint32_t row, const float* v)
+__device__ __forceinline__ void store_chunk(uint8_t* tile, uint32_t row, uint32_t chunk, const float* v)
 {
+    float x[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        float x[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) x[k] = kRelu ? fmaxf(v[8 * c + k], 0.0f) : v[8 * c + k];
-        uint4 w;
-        w.x = pack_bf16(x[0], x[1]); w.y = pack_bf16(x[2], x[3]);
-        w.z = pack_bf16(x[4], x[5]); w.w = pack_bf16(x[6], x[7]);
-        *reinterpret_cast<uint4*>(tile + swz(row, c)) = w;
-    }
+    for (int k = 0; k < 8; ++k) x[k] = kRelu ? fmaxf(v[k], 0.0f) : v[k];
+    uint4 w;
+    w.x = pack_bf16(x[0], x[1]); w.y = pack_bf16(x[2], x[3]);
+    w.z = pack_bf16(x[4], x[5]); w.w = pack_bf16(x[6], x[7]);
+    *reinterpret_cast<uint4*>(tile + swz(row, chunk)) = w;
 }
 
 // ---------------------------------------------------------------- PTX wrappers
@@ -209,6 +217,20 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v)
         : "memory");
 #pragma unroll
     for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
+}
+
+// The same of 8 columns.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v)
+{
+    uint32_t r[8];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[k]);
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)

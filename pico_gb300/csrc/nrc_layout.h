@@ -57,7 +57,19 @@ struct GridGeometry {
     uint32_t table_mask;             // entries per level - 1 (a power of two)
     uint32_t log2_table;
     float lo[3], inv_extent[3];      // position normalisation to the unit cube
+    // the replicated levels' places in a copy of their gradients (kNoReplica: not replicated), and its entries
+    uint32_t rep_base[kLevels];
+    uint32_t rep_entries;
 };
+
+// The coarse levels' gradients.  A training batch's records fall into a few dozen cells of the coarsest levels, and
+// their atomics queue at the same addresses: of the training kernel's 240 us for 65,536 records on the surfaces of a
+// room, levels 0 to 3 took 88, 4 to 7 24, 8 to 15 19, the rest 69.  So the dense levels of at most kReplicaMax entries
+// gather in kReplicas copies, one for every kReplicas-th CTA, which gather_gradients_kernel sums: 143 us (16 copies 142,
+// 32 145, 4 160; copies of up to 2^19 entries 134, lost again in clearing them), the step's fetch included 690 -> 614 us.
+// Smaller batches queue less, and clearing and summing the copies costs some 5 us.
+constexpr uint32_t kNoReplica = 0xffffffffu, kReplicaMax = 1u << 17, kReplicaRecords = 1u << 14;
+constexpr int kReplicas = 8;
 
 }  // namespace nrc
 }  // namespace pico
