@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kRenderThreads) raygen_kernel(PathBatch b, Cam
             b.ior_lo[i] = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
         }
         uint32_t at, unused;
-        block_append(r, live, &b.counters[0], false, nullptr, app, at, unused);
+        block_append(r, live, &b.depths[0].paths, false, nullptr, app, at, unused);
         if (live) b.queue[0][at] = i;
     }
 }
@@ -295,7 +295,8 @@ __global__ void __launch_bounds__(kRenderThreads, kShadeBlocksPerSm) shade_kerne
                                                               uint32_t max_depth, bool trace_last)
 {
     __shared__ AppendScratch app;
-    const uint32_t n = b.counters[cur];
+    const uint32_t n = b.depths[depth % kDepthRing].paths;
+    DepthQueues* next = b.depths + (depth + 1) % kDepthRing;
     const uint32_t nxt = cur ^ 1;
     // whole blocks iterate together so the queue appends can use block collectives
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -422,7 +423,7 @@ __global__ void __launch_bounds__(kRenderThreads, kShadeBlocksPerSm) shade_kerne
             }
         }
         uint32_t at, sat;
-        block_append(r, cont, &b.counters[nxt], shadow, &b.counters[2], app, at, sat);
+        block_append(r, cont, &next->paths, shadow, &next->shadows, app, at, sat);
         if (cont) b.queue[nxt][at] = i;
         if (shadow) b.shadow_queue[sat] = i;
     }
@@ -459,7 +460,8 @@ __global__ void __launch_bounds__(kRenderThreads, kShadeBlocksPerSm) shade_physi
 {
     using namespace phys;
     __shared__ AppendScratch app;
-    const uint32_t n = b.counters[cur];
+    const uint32_t n = b.depths[depth % kDepthRing].paths;
+    DepthQueues* next = b.depths + (depth + 1) % kDepthRing;
     const uint32_t nxt = cur ^ 1;
     const uint32_t nl = sc.nlights + (sc.use_sun ? 1u : 0u);
     const float4* light_geo = reinterpret_cast<const float4*>(sc.light_tri_geo);
@@ -668,7 +670,7 @@ __global__ void __launch_bounds__(kRenderThreads, kShadeBlocksPerSm) shade_physi
             }
         }
         uint32_t at, sat;
-        block_append(r, cont, &b.counters[nxt], shadow, &b.counters[2], app, at, sat);
+        block_append(r, cont, &next->paths, shadow, &next->shadows, app, at, sat);
         if (cont) b.queue[nxt][at] = i;
         if (shadow) b.shadow_queue[sat] = i;
         if (nrc.mode != kNrcOff) {
@@ -711,7 +713,7 @@ __global__ void __launch_bounds__(kRenderThreads) train_raygen_kernel(PathBatch 
             b.depth[i] = 0;
         }
         uint32_t at, unused;
-        block_append(r, live, &b.counters[0], false, nullptr, app, at, unused);
+        block_append(r, live, &b.depths[0].paths, false, nullptr, app, at, unused);
         if (live) b.queue[0][at] = i;
     }
 }
@@ -973,7 +975,7 @@ static unsigned extend_grid(uint32_t ctas_per_sm)
 // One closest-hit launch; with counters, the counting variant (128 threads per CTA).
 template <int kOrder>
 static void launch_extend(const SceneView& sc, PathBatch& b, const uint32_t* q, const uint32_t* count,
-                          const uint32_t* sq, const uint32_t* scount, DeviceStatus* status,
+                          const uint32_t* sq, const uint32_t* scount, unsigned long long* work, DeviceStatus* status,
                           unsigned long long* tally, unsigned long long* counters, cudaStream_t st)
 {
     unsigned long long* stally = &status->rays[2];
@@ -982,26 +984,26 @@ static void launch_extend(const SceneView& sc, PathBatch& b, const uint32_t* q, 
     // block shape asked for
     if (counters) {
         extend_kernel<kOrder | kBounded, 128, true><<<extend_grid<kOrder | kBounded, 128, true>(b.extend_ctas), 128,
-                                                     0, st>>>(sc, b, q, count, sq, scount, &status->work,
+                                                     0, st>>>(sc, b, q, count, sq, scount, work,
                                                               &status->trace_error, tally, stally, counters);
         return;
     }
     if constexpr ((kOrder & (kBounded | kWatertight)) != 0) {
         extend_kernel<kOrder, 128><<<extend_grid<kOrder, 128>(b.extend_ctas), 128, 0, st>>>(
-            sc, b, q, count, sq, scount, &status->work, &status->trace_error, tally, stally, nullptr);
+            sc, b, q, count, sq, scount, work, &status->trace_error, tally, stally, nullptr);
     } else {
         switch (b.extend_threads) {
         case 64:
             extend_kernel<kOrder, 64><<<extend_grid<kOrder, 64>(b.extend_ctas), 64, 0, st>>>(
-                sc, b, q, count, sq, scount, &status->work, &status->trace_error, tally, stally, nullptr);
+                sc, b, q, count, sq, scount, work, &status->trace_error, tally, stally, nullptr);
             break;
         case 256:
             extend_kernel<kOrder, 256><<<extend_grid<kOrder, 256>(b.extend_ctas), 256, 0, st>>>(
-                sc, b, q, count, sq, scount, &status->work, &status->trace_error, tally, stally, nullptr);
+                sc, b, q, count, sq, scount, work, &status->trace_error, tally, stally, nullptr);
             break;
         default:
             extend_kernel<kOrder, 128><<<extend_grid<kOrder, 128>(b.extend_ctas), 128, 0, st>>>(
-                sc, b, q, count, sq, scount, &status->work, &status->trace_error, tally, stally, nullptr);
+                sc, b, q, count, sq, scount, work, &status->trace_error, tally, stally, nullptr);
         }
     }
 }
@@ -1061,20 +1063,20 @@ static cudaError_t run_depth_loop(const SceneView& sc, PathBatch& b, uint32_t ma
         sc.sky_kind != PICO_SKY_CONSTANT || sc.sky[0] != 0.0f || sc.sky[1] != 0.0f || sc.sky[2] != 0.0f;
     int cur = 0;
     for (uint32_t depth = 0; depth <= max_depth; ++depth) {
-        e = cudaMemsetAsync(&status->work, 0, sizeof(unsigned long long), st);
-        if (e != cudaSuccess) return e;
+        DepthQueues* const here = b.depths + depth % kDepthRing;
+        if (depth + 1 >= kDepthRing) {
+            e = cudaMemsetAsync(b.depths + (depth + 1) % kDepthRing, 0, sizeof(DepthQueues), st);
+            if (e != cudaSuccess) return e;
+        }
         unsigned long long* tally = &status->rays[depth == 0 ? 0 : 1];
         // this depth's segments, and from depth 1 on the previous shade's shadow rays
         const uint32_t* sq = depth > 0 ? b.shadow_queue : nullptr;
         if (timer && (e = timer->record(st)) != cudaSuccess) return e;
         with_variant(order, sc, [&](auto v) {
-            launch_extend<decltype(v)::value>(sc, b, b.queue[cur], &b.counters[cur], sq, &b.counters[2], status,
-                                              tally, counters, st);
+            launch_extend<decltype(v)::value>(sc, b, b.queue[cur], &here->paths, sq, &here->shadows, &here->work,
+                                              status, tally, counters, st);
         });
         if (timer && (e = timer->record(st)) != cudaSuccess) return e;
-        e = cudaMemsetAsync(&b.counters[cur ^ 1], 0, sizeof(uint32_t), st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(&b.counters[2], 0, sizeof(uint32_t), st);
-        if (e != cudaSuccess) return e;
         if (shade_timer && (e = shade_timer->record(st)) != cudaSuccess) return e;
         if (physical)
             shade_physical_kernel<<<grid_for(shade_physical_kernel, b.n, kRenderThreads), kRenderThreads, 0, st>>>(sc, b, cur, depth,
@@ -1095,7 +1097,7 @@ cudaError_t launch_training_paths(const SceneView& sc, PathBatch& b, const Camer
 {
     PathBatch t = b;
     t.n = n;
-    cudaError_t e = cudaMemsetAsync(t.counters, 0, 4 * sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(t.depths, 0, kDepthRing * sizeof(DepthQueues), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(nrc.count, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     train_raygen_kernel<<<grid_for(train_raygen_kernel, n, kRenderThreads), kRenderThreads, 0, st>>>(t, cam, seed, frame, W, W * H);
@@ -1116,7 +1118,7 @@ cudaError_t launch_render_batch(const SceneView& sc, PathBatch& b, const CameraV
     NrcShadeArgs off{};
     off.mode = kNrcOff;
     const NrcShadeArgs& na = nrc ? *nrc : off;
-    cudaError_t e = cudaMemsetAsync(b.counters, 0, 4 * sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(b.depths, 0, kDepthRing * sizeof(DepthQueues), st);
     if (e == cudaSuccess && na.mode != kNrcOff) e = cudaMemsetAsync(na.count, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     raygen_kernel<<<grid_for(raygen_kernel, b.n, kRenderThreads), kRenderThreads, 0, st>>>(b, cam, seed, physical);

@@ -59,6 +59,15 @@ struct RoundPlan {
     uint32_t pad[3];
 };
 
+// The queue sizes of one depth: its path segments, the shadow rays the shade before it left, and the closest-hit
+// launch's claims.  A batch has a ring of kDepthRing of them, cleared in one go before it starts (a depth beyond the
+// ring clears its own), so that a depth needs no clearing between its launches.
+struct DepthQueues {
+    uint32_t paths, shadows;
+    unsigned long long work;
+};
+constexpr uint32_t kDepthRing = 64;
+
 // Structure-of-arrays path state of one batch (capacity >= n) and the
 // per-pixel accumulation buffers of the whole image.
 struct PathBatch {
@@ -75,7 +84,7 @@ struct PathBatch {
     float4* sorg; float4* sdir; float4* scontrib; float4* senergy;
     uint32_t* queue[2];
     uint32_t* shadow_queue;
-    uint32_t* counters;                // [0], [1]: path queues, [2]: shadow queue
+    DepthQueues* depths;               // queue sizes of depth d at d % kDepthRing
     // image state (W*H entries)
     float* pixels; float* variance; uint32_t* count; uint32_t* taken; uint32_t* done;
     unsigned long long* sample_tally;  // samples added to the image (set by launch_render_batch)

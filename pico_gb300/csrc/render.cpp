@@ -91,7 +91,7 @@ cudaError_t reserve_paths(RenderBuffers& r, size_t n)
     for (DeviceBuffer* b : {&r.hit_tri, &r.depth, &r.ior_n, &r.q0, &r.q1, &r.sq})
         if (e == cudaSuccess) e = b->reserve(n * sizeof(uint32_t));
     if (e == cudaSuccess) e = r.rng.reserve(n * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = r.counters.reserve(4 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = r.counters.reserve(kDepthRing * sizeof(DepthQueues));
     return e;
 }
 
@@ -106,7 +106,7 @@ PathBatch make_batch(RenderBuffers& r, uint32_t n, uint32_t npix, uint32_t W, co
     b.ior_n = as<uint32_t>(r.ior_n); b.ior_lo = as<float4>(r.ior_lo); b.ior_hi = as<float4>(r.ior_hi);
     b.sorg = as<float4>(r.sorg); b.sdir = as<float4>(r.sdir); b.scontrib = as<float4>(r.scontrib);
     b.senergy = as<float4>(r.senergy); b.queue[0] = as<uint32_t>(r.q0); b.queue[1] = as<uint32_t>(r.q1);
-    b.shadow_queue = as<uint32_t>(r.sq); b.counters = as<uint32_t>(r.counters);
+    b.shadow_queue = as<uint32_t>(r.sq); b.depths = as<DepthQueues>(r.counters);
     b.pixels = as<float>(r.pixels); b.variance = as<float>(r.variance); b.count = as<uint32_t>(r.count);
     b.taken = as<uint32_t>(r.taken); b.done = as<uint32_t>(r.done);
     return b;

@@ -38,25 +38,25 @@ __device__ __forceinline__ void write_hit(const SceneView& sc, const TraceHit& h
 
 // The rays of a batch for walk_queue: a lane's tag is the ray's index.
 struct BatchRays {
-    using Tag = uint64_t;
-    using Index = uint64_t;
+    using Tag = uint32_t;
+    using Index = uint32_t;   // launch_trace cuts longer batches
     const SceneView& sc;
     const float4* rays;
     pico_hit* hits;
     DeviceStatus* status;
 
-    __device__ __forceinline__ uint64_t load(uint64_t k, float4& o, float4& d, float& tmax, float& exit_below,
+    __device__ __forceinline__ uint32_t load(uint32_t k, float4& o, float4& d, float& tmax, float& exit_below,
                                              bool& occlusion) const
     {
-        o = __ldg(rays + 2 * k);
-        d = __ldg(rays + 2 * k + 1);
+        o = __ldg(rays + 2 * (size_t)k);
+        d = __ldg(rays + 2 * (size_t)k + 1);
         tmax = INFINITY;
         exit_below = -INFINITY;
         occlusion = false;
         return k;
     }
 
-    __device__ __forceinline__ void finish(uint64_t tag, const TraceHit& h, int s) const
+    __device__ __forceinline__ void finish(uint32_t tag, const TraceHit& h, int s) const
     {
         if (s != kTraceOk) atomicOr(&status->trace_error, s);
         write_hit(sc, h, s, hits + tag);
@@ -65,7 +65,7 @@ struct BatchRays {
 
 template <bool kCount, int kOrder>
 __global__ void __launch_bounds__(kTraceThreads, trace_min_blocks<kOrder>())
-    trace_kernel(SceneView sc, const float4* __restrict__ rays, uint64_t n, pico_hit* __restrict__ hits,
+    trace_kernel(SceneView sc, const float4* __restrict__ rays, uint32_t n, pico_hit* __restrict__ hits,
                  DeviceStatus* status)
 {
     TraceCounters cnt{0, 0, 0, 0};
@@ -123,7 +123,7 @@ int resident_blocks(const void* kernel, int threads)
 }
 
 template <bool kCount, int kOrder>
-static cudaError_t launch_trace_t(const SceneView& sc, const float4* r, uint64_t n, pico_hit* hits,
+static cudaError_t launch_trace_t(const SceneView& sc, const float4* r, uint32_t n, pico_hit* hits,
                                   DeviceStatus* status, cudaStream_t stream)
 {
     static int per_sm = 0;
@@ -134,7 +134,7 @@ static cudaError_t launch_trace_t(const SceneView& sc, const float4* r, uint64_t
         if (per_sm < 1) per_sm = 1;
     }
     uint64_t blocks = (uint64_t)sm_count() * (uint64_t)per_sm;
-    const uint64_t needed = (n + kTraceThreads - 1) / kTraceThreads;
+    const uint64_t needed = (n + kTraceThreads / 32 - 1) / (kTraceThreads / 32);   // down to one ray per warp
     if (blocks > needed) blocks = needed;
     trace_kernel<kCount, kOrder><<<(unsigned)blocks, kTraceThreads, 0, stream>>>(sc, r, n, hits, status);
     return cudaGetLastError();
@@ -143,15 +143,23 @@ static cudaError_t launch_trace_t(const SceneView& sc, const float4* r, uint64_t
 cudaError_t launch_trace(const SceneView& sc, const pico_ray* rays, uint64_t n, pico_hit* hits,
                          DeviceStatus* status, bool count, int order, cudaStream_t stream)
 {
-    cudaError_t e = cudaMemsetAsync(&status->work, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess || n == 0) return e;
-    const float4* r = reinterpret_cast<const float4*>(rays);
-    return with_variant(order, sc, [&](auto v) {
-        constexpr int V = decltype(v)::value;
-        // the counting variant (measurement only) always reads the bounds at run time
-        return count ? launch_trace_t<true, V | kBounded>(sc, r, n, hits, status, stream)
-                     : launch_trace_t<false, V>(sc, r, n, hits, status, stream);
-    });
+    if (n == 0) return cudaMemsetAsync(&status->work, 0, sizeof(unsigned long long), stream);
+    // the kernel's ray indices are 32 bits (56 registers hold a walk without spills then), so a longer batch is cut
+    constexpr uint64_t kMost = 1ull << 31;
+    for (uint64_t at = 0; at < n; at += kMost) {
+        const uint32_t m = (uint32_t)(n - at < kMost ? n - at : kMost);
+        cudaError_t e = cudaMemsetAsync(&status->work, 0, sizeof(unsigned long long), stream);
+        if (e != cudaSuccess) return e;
+        const float4* r = reinterpret_cast<const float4*>(rays + at);
+        e = with_variant(order, sc, [&](auto v) {
+            constexpr int V = decltype(v)::value;
+            // the counting variant (measurement only) always reads the bounds at run time
+            return count ? launch_trace_t<true, V | kBounded>(sc, r, m, hits + at, status, stream)
+                         : launch_trace_t<false, V>(sc, r, m, hits + at, status, stream);
+        });
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace pico

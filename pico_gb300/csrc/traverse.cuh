@@ -743,9 +743,15 @@ __device__ __forceinline__ int nf_rare(NearFirstState& w, const SceneView& sc, u
 // 7 % slower than waiting, warps that held their 32 rays until the slowest ended another
 // 4.4 %, claims of 32 entries with one atomic per refill 4.8 %.
 //
-// A launch with fewer than kBigLaunch rays per warp claims 32 entries at a time, so that
-// its rays spread over the warps (the Cornell box at 256 x 256 has a few dozen rays per
-// warp and launch).  A 32-bit Index suffices for queues of fewer than 2^32 entries.
+// A launch with fewer than kBigLaunch rays per warp claims 32 entries at a time, and one
+// with fewer than 32 gives every warp its share of them, one ray each at least: such
+// launches (a render's late depths, training paths, small batches) take as long as their
+// longest ray, which walks faster with fewer others in its warp, and every warp's first
+// claim is its own, without the counter.  Against claims of at least 32 from the counter,
+// with the clearing between a depth's launches gone too (DepthQueues): Cornell box at
+// 256 x 256 1.23 -> 1.16 ms, a radiance-cache preview of 960 x 540 10.4 -> 9.1 ms, 1000 rays
+// 46.7 -> 44.1 us with the host's wait; shares of 4 or 8 rays at least 9.6 and 9.8 ms for
+// the preview.
 constexpr int kReleaseWait = 5;   // of 8 walking lanes
 constexpr int kInnerMoves = 2;
 constexpr uint32_t kRefillIdle = 8;
@@ -754,6 +760,8 @@ constexpr uint32_t kClaim = 64;   // queue entries a warp claims at a time
 // could run backwards and the warp would never claim again.
 static_assert(kClaim >= 32, "a claim covers a whole warp's refill");
 constexpr uint32_t kBigLaunch = 1024;   // rays per warp from which a launch claims kClaim at a time
+__device__ __forceinline__ uint32_t walk_warps() { return gridDim.x * (blockDim.x >> 5); }
+
 template <bool kCount, bool kImplicit, bool kRuntimeBounds, bool kWT, class Rays>
 __device__ __forceinline__ void walk_queue(const SceneView& sc, Rays& rays, typename Rays::Index n,
                                            unsigned long long* work, TraceCounters* cnt)
@@ -766,12 +774,15 @@ __device__ __forceinline__ void walk_queue(const SceneView& sc, Rays& rays, type
     int status = kIdle;
     unsigned busy = 0;   // warp-uniform: the lanes that were walking at the last release
     bool more = true;    // warp-uniform: the queue may hold entries
-    Index next = 0, end = 0;   // warp-uniform: the warp's claimed entries [next, end)
-    // a launch with fewer than kBigLaunch rays per warp claims 32 at a time, so that its rays spread over the warps
-    const bool big = (uint64_t)n >= (uint64_t)gridDim.x * (blockDim.x >> 5) * kBigLaunch;
-    const uint32_t claim = big ? kClaim : 32u;
+    const uint64_t share = ((uint64_t)n + walk_warps() - 1) / walk_warps();   // rays per warp
+    const uint32_t claim = share >= kBigLaunch ? kClaim : (share > 32 ? 32u : (uint32_t)share);
+    // a warp's first claim is its own, without the counter; a warp beyond the launch's rays has nothing to do
+    Index next = (Index)((uint64_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * claim);
+    uint32_t avail = claim;   // warp-uniform: the warp's claimed entries are [next, next + avail)
+    if (next >= n) return;
+    const int refill = claim >= 32 ? 32 - (int)kRefillIdle : (claim > kRefillIdle ? (int)(claim - kRefillIdle) : 0);
     for (;;) {
-        if (more ? __popc(busy) <= 32 - kRefillIdle : busy == 0) {
+        if (more ? __popc(busy) <= refill : busy == 0) {
             if (status >= 0) {
                 const TraceHit best{mem_float(mem, kMemT), mem[kMemRank], mem[kMemTri], mem_float(mem, kMemU),
                                     mem_float(mem, kMemV)};
@@ -779,14 +790,15 @@ __device__ __forceinline__ void walk_queue(const SceneView& sc, Rays& rays, type
                 status = kIdle;
             }
             if (!more) break;
-            const unsigned idle = ~busy;
+            // the lanes that take rays: all, or as many as the launch has rays per warp
+            const unsigned idle = ~busy & (claim >= 32 ? 0xffffffffu : (1u << claim) - 1u);
             const uint32_t need = __popc(idle);
-            const uint32_t avail = (uint32_t)(end - next);
             Index fresh = 0;
-            if (need > avail) {
+            const bool fetch = need > avail;
+            if (fetch) {
                 unsigned long long base = 0;
                 if (lane == 0) base = atomicAdd(work, (unsigned long long)claim);
-                base = __shfl_sync(0xffffffffu, base, 0);
+                base = __shfl_sync(0xffffffffu, base, 0) + (unsigned long long)walk_warps() * claim;
                 if (base >= (unsigned long long)n) {
                     more = false;
                     fresh = n;
@@ -796,12 +808,6 @@ __device__ __forceinline__ void walk_queue(const SceneView& sc, Rays& rays, type
             }
             const uint32_t r = __popc(idle & ((1u << lane) - 1u));
             const Index k = r < avail ? next + r : fresh + (r - avail);
-            if (need > avail) {
-                next = fresh + (need - avail);
-                end = fresh + claim;
-            } else {
-                next += need;
-            }
             if (((idle >> lane) & 1u) && k < n && (r < avail || more)) {
                 float4 o, d;
                 float tmax, exit_below;
@@ -809,6 +815,13 @@ __device__ __forceinline__ void walk_queue(const SceneView& sc, Rays& rays, type
                 tag = rays.load(k, o, d, tmax, exit_below, occlusion);
                 nf_start<kWT>(w, mem, sc, o, d, tmax, exit_below, occlusion);
                 status = kWalking;
+            }
+            if (fetch) {
+                next = fresh + (need - avail);
+                avail = claim - (need - avail);
+            } else {
+                next += need;
+                avail -= need;
             }
             busy = __ballot_sync(0xffffffffu, status == kWalking);
             if (busy == 0) continue;

@@ -54,3 +54,16 @@ def test_tile_order_covers_ragged_images(ctx, size):
     assert (count == 6).all() and (items[0]["sample_count"] == 6).all()
     np.testing.assert_array_equal(whole, chunked)
     np.testing.assert_array_equal(whole, items[0]["pixels"])
+
+
+@pytest.mark.parametrize("n", [1, 5, 31, 33, 1000, 5471, 5472, 5473, 20000, 175104, 175105])
+def test_few_rays_per_warp(ctx, oracle, n):
+    """Launches of one ray per warp up to 32: every ray is walked once, whatever the warps' shares."""
+    s = scenes.instance_field(n_instances=16, level=1, seed=3, extent=5.0)
+    rays = scenes.surface_rays(s, n, seed=n)
+    gs = ctx.upload(s)
+    got, want = gs.trace_closest(rays), oracle.scene(s).trace(rays)
+    gs.free()
+    for k in ("inst", "prim"):
+        np.testing.assert_array_equal(got[k], want[k])
+    np.testing.assert_array_equal(got["t"].view(np.uint32), want["t"].view(np.uint32))
