@@ -71,7 +71,6 @@ struct Params {
 struct Prepared {
     uint32_t W = 0, H = 0;
     size_t npx = 0, nactive = 0;
-    uint64_t samples_before = 0;
     CameraView cam{};
 };
 
@@ -159,7 +158,8 @@ cudaError_t ensure_state(pico_gpu_ctx* ctx, uint32_t nrenders, size_t npieces, u
     return e;
 }
 
-// Uploads one render's progressive buffers and active-pixel list into its image slot.
+// Uploads one render's progressive buffers into its image slot and lists its active pixels: on the device when every
+// pixel is active, else here.  A fresh render's mean and variance are not uploaded (CountScan).
 cudaError_t upload_render(const pico_render_item& it, BatchSlot& s, Prepared& pr, cudaStream_t st,
                           std::vector<uint32_t>& active, std::vector<uint32_t>& done)
 {
@@ -168,28 +168,34 @@ cudaError_t upload_render(const pico_render_item& it, BatchSlot& s, Prepared& pr
     pr.W = cfg.width;
     pr.H = cfg.height;
     pr.npx = (size_t)pr.W * pr.H;
-    active.clear();
-    done.assign(pr.npx, 0u);
-    pr.samples_before = 0;
-    for_tile_pixels(pr.W, pr.H, [&](uint32_t px) {
-        pr.samples_before += it.sample_count[px];
-        if (it.sample_count[px] >= cfg.max_samples) done[px] = 1;
-        else active.push_back(px);
-    });
-    pr.nactive = active.size();
+    const CountScan scan = scan_counts(it.sample_count, pr.npx, cfg.max_samples);
+    pr.nactive = scan.unfinished;
     pr.cam = make_camera_view(it.camera);
     cudaError_t e = r.pixels.reserve(pr.npx * 3 * sizeof(float));
     if (e == cudaSuccess) e = r.variance.reserve(pr.npx * 3 * sizeof(float));
     for (DeviceBuffer* b : {&r.count, &r.taken, &r.done, &r.pix_list})
         if (e == cudaSuccess) e = b->reserve(pr.npx * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r.pixels.ptr, it.pixels_rgb, pr.npx * 3 * sizeof(float),
-                                              cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r.variance.ptr, it.variance_rgb, pr.npx * 3 * sizeof(float),
-                                              cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r.count.ptr, it.sample_count, pr.npx * sizeof(uint32_t),
-                                              cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r.done.ptr, done.data(), pr.npx * sizeof(uint32_t),
-                                              cudaMemcpyHostToDevice, st);
+    if (scan.fresh) {
+        if (e == cudaSuccess) e = cudaMemsetAsync(r.count.ptr, 0, pr.npx * sizeof(uint32_t), st);
+    } else {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(r.pixels.ptr, it.pixels_rgb, pr.npx * 3 * sizeof(float),
+                                                  cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(r.variance.ptr, it.variance_rgb, pr.npx * 3 * sizeof(float),
+                                                  cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(r.count.ptr, it.sample_count, pr.npx * sizeof(uint32_t),
+                                                  cudaMemcpyHostToDevice, st);
+    }
+    if (e != cudaSuccess) return e;
+    if (pr.nactive == pr.npx)
+        return launch_prepare_image(as<uint32_t>(r.count), pr.W, pr.H, cfg.max_samples, as<uint32_t>(r.pix_list),
+                                    as<uint32_t>(r.done), as<uint32_t>(r.taken), st);
+    active.clear();
+    done.assign(pr.npx, 0u);
+    for_tile_pixels(pr.W, pr.H, [&](uint32_t px) {
+        if (it.sample_count[px] >= cfg.max_samples) done[px] = 1;
+        else active.push_back(px);
+    });
+    e = cudaMemcpyAsync(r.done.ptr, done.data(), pr.npx * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(r.taken.ptr, 0, pr.npx * sizeof(uint32_t), st);
     if (e == cudaSuccess && pr.nactive)
         e = cudaMemcpyAsync(r.pix_list.ptr, active.data(), pr.nactive * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
@@ -400,6 +406,11 @@ int run_batch(pico_gpu_ctx* ctx, uint32_t n, const pico_render_item* items, cons
     }
     const auto t_run = clock::now();
     e = cudaGraphLaunch(exec, st);
+    for (uint32_t r = 0; r < n && e == cudaSuccess; ++r) {   // while the graph runs
+        populate_for_writing(items[r].pixels_rgb, prep[r].npx * 3 * sizeof(float));
+        populate_for_writing(items[r].variance_rgb, prep[r].npx * 3 * sizeof(float));
+        populate_for_writing(items[r].sample_count, prep[r].npx * sizeof(uint32_t));
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     const auto t_end = clock::now();
     cleanup();
@@ -418,6 +429,7 @@ int run_batch(pico_gpu_ctx* ctx, uint32_t n, const pico_render_item* items, cons
     for (size_t j = 0; j < np; ++j) {
         const DeviceStatus& ds = status[j];
         rays += ds.rays[0] + ds.rays[1] + ds.rays[2];
+        samples += ds.rays[3];   // what accumulate added
         const uint32_t r = pieces[j].render;
         if (ds.trace_error && result == PICO_OK)
             result = set_error(ctx, (ds.trace_error & kTraceStackOverflow) ? PICO_ERR_STACK_OVERFLOW : PICO_ERR_TIMEOUT,
@@ -433,12 +445,8 @@ int run_batch(pico_gpu_ctx* ctx, uint32_t n, const pico_render_item* items, cons
                                                   cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(it.sample_count, s.r.count.ptr, pr.npx * sizeof(uint32_t),
                                                   cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) break;
-        uint64_t after = 0;
-        for (size_t px = 0; px < pr.npx; ++px) after += it.sample_count[px];
-        samples += after - pr.samples_before;
     }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(ctx, e, "batch download");
     if (rep) {
         rep->build_ms = std::chrono::duration<double, std::milli>(t_run - t_build).count();

@@ -1,5 +1,10 @@
 // The C ABI of libpico_gpu (include/pico_gpu.h): contexts, scene upload and
 // the closest-hit entry points.  Rendering and denoising live in render.cpp.
+#include <cerrno>
+#ifdef __linux__
+#include <sys/mman.h>
+#include <unistd.h>
+#endif
 #include "capi_internal.h"
 
 #include <cuda.h>   // driver types for cuPointerGetAttribute (resolved at run time, not linked)
@@ -23,6 +28,22 @@ int cuda_error(pico_gpu_ctx* ctx, cudaError_t e, const char* what)
     if (e == cudaErrorMemoryAllocation)
         return set_error(ctx, PICO_ERR_OUT_OF_MEMORY, std::string(what) + ": " + cudaGetErrorString(e));
     return set_error(ctx, PICO_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+void populate_for_writing(void* p, size_t bytes)
+{
+#ifdef __linux__
+    constexpr int kPopulateWrite = 23;   // MADV_POPULATE_WRITE (Linux 5.14)
+    if (!p || bytes < (size_t(1) << 16)) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(p) & ~(page - 1), hi = reinterpret_cast<uintptr_t>(p) + bytes;
+    const int kept = errno;
+    (void)madvise(reinterpret_cast<void*>(lo), hi - lo, kPopulateWrite);
+    errno = kept;
+#else
+    (void)p;
+    (void)bytes;
+#endif
 }
 
 cudaError_t DeviceBuffer::reserve(size_t bytes)
@@ -509,6 +530,7 @@ int pico_gpu_trace_closest(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const
         e = cudaMemcpyAsync(dr, rays + off, m * sizeof(pico_ray), cudaMemcpyHostToDevice, streams[s]);
         if (e == cudaSuccess)
             e = launch_trace(traversal_view(ctx, scene), dr, m, dh, s ? ctx->status2() : ctx->status, false, scene_order(ctx, scene), streams[s]);
+        populate_for_writing(hits + off, m * sizeof(pico_hit));   // while the chunk is traversed
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(hits + off, dh, m * sizeof(pico_hit), cudaMemcpyDeviceToHost, streams[s]);
     }

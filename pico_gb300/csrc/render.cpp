@@ -95,6 +95,17 @@ cudaError_t reserve_paths(RenderBuffers& r, size_t n)
     return e;
 }
 
+CountScan scan_counts(const uint32_t* count, size_t npx, uint32_t max_samples)
+{
+    size_t unfinished = 0;
+    uint32_t any = 0;
+    for (size_t p = 0; p < npx; ++p) {
+        unfinished += count[p] < max_samples ? 1u : 0u;
+        any |= count[p];
+    }
+    return CountScan{unfinished, npx > 0 && any == 0 && max_samples > 0};
+}
+
 PathBatch make_batch(RenderBuffers& r, uint32_t n, uint32_t npix, uint32_t W, const uint32_t* pix_list)
 {
     PathBatch b{};
@@ -183,6 +194,7 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
         PathBatch tb = make_batch(r, ntrain, 0, W, nullptr);
         cudaError_t te = launch_training_paths(traversal_view(ctx, scene), tb, cam, train_seed, (uint32_t)c->train_passes, ntrain,
                                                W, H, max_depth, na, as<float4>(r.nrc_tgt), ctx->status, order, st);
+        r.populate_results();
         uint32_t nrec = 0;
         if (te == cudaSuccess) te = cudaMemcpyAsync(&nrec, na.count, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
         if (te == cudaSuccess) te = cudaStreamSynchronize(st);
@@ -220,6 +232,7 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
             PathBatch b = make_batch(r, npix, npix, W, as<uint32_t>(r.pix_list) + p0);
             e = launch_render_batch(traversal_view(ctx, scene), b, cam, cfg->seed, 1, max_depth, cfg->max_samples,
                                     cfg->max_variance, PICO_ESTIMATOR_RADIANCE_CACHE, ctx->status, order, st, &na);
+            r.populate_results();
             uint32_t nq = 0;
             if (e == cudaSuccess) e = cudaMemcpyAsync(&nq, na.count, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -309,6 +322,7 @@ static int run_exit_aware_rounds(pico_gpu_ctx* ctx, const pico_gpu_scene* scene,
                                 nullptr, pp);
         if (e == cudaSuccess && k + 1 < rounds)
             e = launch_compact_pixels(plan, lists[k & 1], as<uint32_t>(r.done), lists[(k + 1) & 1], nactive, st);
+        r.populate_results();
         if (e == cudaSuccess && should_quit) e = cudaStreamSynchronize(st);
     }
     if (e != cudaSuccess) return cuda_error(ctx, e, "render round");
@@ -346,11 +360,35 @@ int run_sample_batches(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pic
             e = launch_render_batch(traversal_view(ctx, scene), b, cam, cfg->seed, spb, cfg->max_ray_depth, cfg->max_samples,
                                     cfg->max_variance, (int)cfg->estimator, ctx->status, scene_order(ctx, scene), st,
                                     nullptr, pp);
+            r.populate_results();
             if (e == cudaSuccess && should_quit) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) return cuda_error(ctx, e, "render batch");
         }
     }
     return PICO_OK;
+}
+
+// A cancelled render whose mean and variance were not uploaded: the device buffers get the caller's values for the
+// pixels without a sample.
+cudaError_t restore_unsampled(RenderBuffers& r, const float* pixels, const float* variance, size_t npx, cudaStream_t st)
+{
+    std::vector<uint32_t> count(npx);
+    std::vector<float> mean(3 * npx), var(3 * npx);
+    cudaError_t e = cudaMemcpyAsync(count.data(), r.count.ptr, npx * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(mean.data(), r.pixels.ptr, 3 * npx * sizeof(float), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(var.data(), r.variance.ptr, 3 * npx * sizeof(float), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    for (size_t p = 0; p < npx; ++p)
+        if (count[p] == 0)
+            for (size_t k = 3 * p; k < 3 * p + 3; ++k) {
+                mean[k] = pixels[k];
+                var[k] = variance[k];
+            }
+    e = cudaMemcpyAsync(r.pixels.ptr, mean.data(), 3 * npx * sizeof(float), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(r.variance.ptr, var.data(), 3 * npx * sizeof(float), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the host vectors end with this call
+    return e;
 }
 
 // Scene.cpp:212-234 after the samples: the a-trous pass on the G-buffer replaces
@@ -409,25 +447,30 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
         if (e == cudaSuccess) e = b->reserve(npx * sizeof(uint32_t));
     if (e != cudaSuccess) return cuda_error(ctx, e, "image buffers");
 
-    // The radiance cache's passes take the pixels still sampling as a compacted list built
-    // here; the other estimators list every pixel on the device (prepare_image_kernel) and
-    // skip the finished ones there, with no host pass over the image.
-    const bool host_list = cfg->estimator == PICO_ESTIMATOR_RADIANCE_CACHE;
+    // The pixels are listed on the device (prepare_image_kernel), every one of them; the sample batches skip the
+    // finished ones there.  The radiance cache's passes take a compacted list, which is built here when some pixels
+    // are finished.  A fresh render's mean and variance are not uploaded (accumulate replaces them with a pixel's
+    // first sample): the caller's pages, often untouched, are then faulted in once, by the download, instead of twice.
+    const CountScan scan = scan_counts(sample_count, npx, cfg->max_samples);
+    const bool with_cache = cfg->estimator == PICO_ESTIMATOR_RADIANCE_CACHE;
+    const bool host_list = with_cache && scan.unfinished < npx;
     std::vector<uint32_t> active, done;
-    uint64_t samples_before = 0;
     if (host_list) {
         done.assign(npx, 0u);
-        active.reserve(npx);
+        active.reserve(scan.unfinished);
         for_tile_pixels(W, H, [&](uint32_t p) {
-            samples_before += sample_count[p];
             if (sample_count[p] >= cfg->max_samples) done[p] = 1;
             else active.push_back(p);
         });
     }
     for (uint64_t& v : ctx->render_stats) v = 0;
-    e = cudaMemcpyAsync(r.pixels.ptr, pixels, npx * 3 * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r.variance.ptr, variance, npx * 3 * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r.count.ptr, sample_count, npx * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+    if (scan.fresh) {
+        e = cudaMemsetAsync(r.count.ptr, 0, npx * sizeof(uint32_t), st);
+    } else {
+        e = cudaMemcpyAsync(r.pixels.ptr, pixels, npx * 3 * sizeof(float), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(r.variance.ptr, variance, npx * 3 * sizeof(float), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(r.count.ptr, sample_count, npx * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+    }
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->status->rays, 0, sizeof(ctx->status->rays), st);
     if (host_list) {
         if (e == cudaSuccess) e = cudaMemcpyAsync(r.done.ptr, done.data(), npx * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
@@ -444,9 +487,10 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
 
     const CameraView cam = make_camera_view(*camera);
     bool cancelled = false;
-    const size_t nactive = host_list ? active.size() : npx;
+    const size_t nactive = with_cache ? scan.unfinished : npx;
+    r.results = {{pixels, npx * 3 * sizeof(float)}, {variance, npx * 3 * sizeof(float)}, {sample_count, npx * sizeof(uint32_t)}};
     if (nactive > 0 && cfg->max_samples > 0) {
-        status = host_list
+        status = with_cache
                      ? render_with_cache(ctx, scene, ctx->cache, cfg, cam, r, nactive, should_quit, cancelled)
                      : run_sample_batches(ctx, scene, cfg, cam, r, nactive, as<float>(r.pixels),
                                           as<float>(r.variance), as<uint32_t>(r.count), should_quit, st, cancelled);
@@ -454,6 +498,11 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
     }
     status = take_device_status(ctx, st);
     if (status != PICO_OK) return status;
+    if (cancelled && scan.fresh) {
+        // the pixels that took no sample keep the caller's values
+        e = restore_unsampled(r, pixels, variance, npx, st);
+        if (e != cudaSuccess) return cuda_error(ctx, e, "cancelled render");
+    }
     status = finish_image(ctx, scene, cam, cfg, r, as<float>(r.pixels), st);
     if (status != PICO_OK) return status;
 
@@ -464,13 +513,7 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
     if (e == cudaSuccess) e = cudaMemcpyAsync(rays, ctx->status->rays, sizeof(rays), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(ctx, e, "render download");
-    if (host_list) {
-        uint64_t samples_after = 0;
-        for (size_t p = 0; p < npx; ++p) samples_after += sample_count[p];
-        ctx->render_stats[0] = samples_after - samples_before;
-    } else {
-        ctx->render_stats[0] = rays[3];   // the samples accumulate added, tallied on the device
-    }
+    ctx->render_stats[0] = rays[3];   // the samples accumulate added, tallied on the device
     ctx->render_stats[1] = rays[0];
     ctx->render_stats[2] = rays[1];
     ctx->render_stats[3] = rays[2];

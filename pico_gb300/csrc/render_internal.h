@@ -4,6 +4,9 @@
 #include "capi_internal.h"
 #include "kernels_render.h"
 
+#include <utility>
+#include <vector>
+
 // Path state and image buffers of one render, grown on demand.
 struct RenderBuffers {
     pico::DeviceBuffer org, dir, thr, pay, hit, hit_tri, rng, depth, ior_n, ior_lo, ior_hi, sorg, sdir, scontrib,
@@ -16,6 +19,13 @@ struct RenderBuffers {
     // radiance cache: terminal queries / training records, record throughput and
     // payload, targets, previous roughness per path, entry counters
     pico::DeviceBuffer nrc_q, nrc_tp, nrc_tgt, nrc_prev, nrc_count;
+    // the host buffers this render's results will go to, populated once the device has its first work
+    std::vector<std::pair<void*, size_t>> results;
+    void populate_results()
+    {
+        for (const auto& b : results) pico::populate_for_writing(b.first, b.second);
+        results.clear();
+    }
     ~RenderBuffers()
     {
         for (pico::DeviceBuffer* b : {&org, &dir, &thr, &pay, &hit, &hit_tri, &rng, &depth, &ior_n, &ior_lo, &ior_hi,
@@ -39,6 +49,13 @@ constexpr uint32_t kMaxPaths = 1u << 26;
 // Device bytes of path state per path that reserve_paths allocates: eleven float4
 // arrays, six uint32 arrays and the 64-bit random state.
 constexpr size_t kPathStateBytes = 11 * 16 + 6 * 4 + 8;
+
+// What a caller's sample counts say before a render of max_samples per pixel.
+struct CountScan {
+    size_t unfinished = 0;   // pixels that will take samples
+    bool fresh = false;      // no pixel has a sample and all will take one: the mean and variance passed in are not read
+};
+CountScan scan_counts(const uint32_t* count, size_t npx, uint32_t max_samples);
 
 template <class T>
 T* as(DeviceBuffer& b) { return static_cast<T*>(b.ptr); }
