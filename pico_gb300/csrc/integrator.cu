@@ -34,16 +34,6 @@ constexpr int kRenderThreads = 256;
 // estimator) and 1.7 % (physical) faster, with identical images.
 constexpr int kShadeBlocksPerSm = 4;
 
-__device__ __forceinline__ uint32_t warp_append(bool take, uint32_t* counter)
-{
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned mask = __ballot_sync(0xffffffffu, take);
-    uint32_t base = 0;
-    if (lane == (unsigned)(__ffs(mask) - 1) && mask) base = atomicAdd(counter, (uint32_t)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, mask ? __ffs(mask) - 1 : 0);
-    return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
-}
-
 // Queue appends with one atomic per block and queue (a same-address atomic per warp
 // measured as the bound of raygen): each warp's count from a ballot, a prefix over
 // the block's warps in shared memory, one atomicAdd per queue by one thread.  Every
@@ -674,24 +664,35 @@ __global__ void __launch_bounds__(kRenderThreads, kShadeBlocksPerSm) shade_physi
         if (cont) b.queue[nxt][at] = i;
         if (shadow) b.shadow_queue[sat] = i;
         if (nrc.mode != kNrcOff) {
-            const uint32_t ea = warp_append(emit, nrc.count);
-            if (emit && ea < nrc.capacity) {
-                float4* q = nrc.queries + 4 * (size_t)ea;
-                q[0] = eq[0]; q[1] = eq[1]; q[2] = eq[2]; q[3] = eq[3];
-                if (nrc.mode == kNrcRecord) {
-                    nrc.rec_tp[2 * (size_t)ea] = et;
-                    nrc.rec_tp[2 * (size_t)ea + 1] = ep;
+            // an entry in its path's pass: one atomic per pass that the warp's paths belong to
+            const unsigned emits = __ballot_sync(0xffffffffu, emit);
+            if (emit) {
+                const uint32_t pass = nrc.passes > 1 ? i / nrc.pass_paths : 0u;
+                const unsigned peers = nrc.passes > 1 ? __match_any_sync(emits, pass) : emits;
+                const unsigned lane = threadIdx.x & 31u, leader = (unsigned)__ffs(peers) - 1u;
+                uint32_t ea = 0;
+                if (lane == leader) ea = atomicAdd(nrc.count + pass, (uint32_t)__popc(peers));
+                ea = __shfl_sync(peers, ea, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+                if (ea < nrc.capacity) {
+                    const size_t entry = (size_t)pass * nrc.capacity + ea;
+                    float4* q = nrc.queries + 4 * entry;
+                    q[0] = eq[0]; q[1] = eq[1]; q[2] = eq[2]; q[3] = eq[3];
+                    if (nrc.mode == kNrcRecord) {
+                        nrc.rec_tp[2 * entry] = et;
+                        nrc.rec_tp[2 * entry + 1] = ep;
+                    }
                 }
             }
         }
     }
 }
 
-// Pixel-pseudo-random camera paths that train the radiance cache: path j of pass
-// `frame` starts at a uniformly drawn pixel with a jitter over the whole pixel.
+// Pixel-pseudo-random camera paths that train the radiance cache: path j of a pass
+// (its frame: `frame` plus the pass's number here) starts at a uniformly drawn pixel
+// with a jitter over the whole pixel.
 __global__ void __launch_bounds__(kRenderThreads) train_raygen_kernel(PathBatch b, CameraView cam,
                                                                      unsigned long long seed, uint32_t frame,
-                                                                     uint32_t W, uint32_t npx)
+                                                                     uint32_t pass_paths, uint32_t W, uint32_t npx)
 {
     __shared__ AppendScratch app;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(kRenderThreads) train_raygen_kernel(PathBatch 
         const uint32_t i = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
         const bool live = i < b.n;
         if (live) {
-            Pcg32 rng = path_rng(seed, i, frame);
+            Pcg32 rng = path_rng(seed, i % pass_paths, frame + i / pass_paths);
             const uint32_t pixel = rng.next() % npx;
             const float x0 = 2.0f * rng.uniform(), x1 = 2.0f * rng.uniform();
             float4 o, d;
@@ -724,20 +725,23 @@ __global__ void __launch_bounds__(kRenderThreads) train_raygen_kernel(PathBatch 
 __global__ void __launch_bounds__(kRenderThreads) nrc_targets_kernel(const float4* __restrict__ queries,
                                                                     const float4* __restrict__ rec_tp,
                                                                     const float4* __restrict__ pay,
-                                                                    const uint32_t* count, uint32_t capacity,
-                                                                    float4* targets)
+                                                                    const uint32_t* count, uint32_t passes,
+                                                                    uint32_t capacity, float4* targets)
 {
-    const uint32_t n = min(*count, capacity);
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const uint32_t path = __float_as_uint(queries[4 * (size_t)j + 3].y);
-        const float4 T = rec_tp[2 * (size_t)j], P = rec_tp[2 * (size_t)j + 1], F = pay[path];
-        float4 t;
-        t.x = T.x > 0.0f ? (F.x - P.x) / T.x : 0.0f;
-        t.y = T.y > 0.0f ? (F.y - P.y) / T.y : 0.0f;
-        t.z = T.z > 0.0f ? (F.z - P.z) / T.z : 0.0f;
-        t.w = 0.0f;
-        if (!(isfinite(F.x) && isfinite(F.y) && isfinite(F.z))) t.x = __int_as_float(0x7fc00000);
-        targets[j] = t;
+    for (uint32_t p = 0; p < passes; ++p) {
+        const uint32_t n = min(count[p], capacity);
+        for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+            const size_t j = (size_t)p * capacity + k;
+            const uint32_t path = __float_as_uint(queries[4 * j + 3].y);
+            const float4 T = rec_tp[2 * j], P = rec_tp[2 * j + 1], F = pay[path];
+            float4 t;
+            t.x = T.x > 0.0f ? (F.x - P.x) / T.x : 0.0f;
+            t.y = T.y > 0.0f ? (F.y - P.y) / T.y : 0.0f;
+            t.z = T.z > 0.0f ? (F.z - P.z) / T.z : 0.0f;
+            t.w = 0.0f;
+            if (!(isfinite(F.x) && isfinite(F.y) && isfinite(F.z))) t.x = __int_as_float(0x7fc00000);
+            targets[j] = t;
+        }
     }
 }
 
@@ -1091,47 +1095,69 @@ static cudaError_t run_depth_loop(const SceneView& sc, PathBatch& b, uint32_t ma
 }
 
 cudaError_t launch_training_paths(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
-                                  uint32_t frame, uint32_t n, uint32_t W, uint32_t H, uint32_t max_depth,
-                                  const NrcShadeArgs& nrc, float4* targets, DeviceStatus* status, int order,
-                                  cudaStream_t st)
+                                  uint32_t frame, uint32_t W, uint32_t H, uint32_t max_depth, const NrcShadeArgs& nrc,
+                                  float4* targets, DeviceStatus* status, int order, cudaStream_t st)
 {
     PathBatch t = b;
-    t.n = n;
+    t.n = nrc.passes * nrc.pass_paths;
     cudaError_t e = cudaMemsetAsync(t.depths, 0, kDepthRing * sizeof(DepthQueues), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(nrc.count, 0, sizeof(uint32_t), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(nrc.count, 0, nrc.passes * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    train_raygen_kernel<<<grid_for(train_raygen_kernel, n, kRenderThreads), kRenderThreads, 0, st>>>(t, cam, seed, frame, W, W * H);
+    train_raygen_kernel<<<grid_for(train_raygen_kernel, t.n, kRenderThreads), kRenderThreads, 0, st>>>(
+        t, cam, seed, frame, nrc.pass_paths, W, W * H);
     e = run_depth_loop(sc, t, max_depth, true, nrc, status, order, st);
     if (e != cudaSuccess) return e;
     nrc_targets_kernel<<<grid_for(nrc_targets_kernel, nrc.capacity, kRenderThreads), kRenderThreads, 0, st>>>(
-        nrc.queries, nrc.rec_tp, t.pay, nrc.count, nrc.capacity, targets);
+        nrc.queries, nrc.rec_tp, t.pay, nrc.count, nrc.passes, nrc.capacity, targets);
+    return cudaGetLastError();
+}
+
+// A batch's camera rays and depth loop.
+static cudaError_t launch_paths(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
+                                uint32_t max_depth, bool physical, const NrcShadeArgs& nrc, DeviceStatus* status,
+                                int order, cudaStream_t st, const RenderProbe* probe)
+{
+    const cudaError_t e = cudaMemsetAsync(b.depths, 0, kDepthRing * sizeof(DepthQueues), st);
+    if (e != cudaSuccess) return e;
+    raygen_kernel<<<grid_for(raygen_kernel, b.n, kRenderThreads), kRenderThreads, 0, st>>>(b, cam, seed, physical);
+    return run_depth_loop(sc, b, max_depth, physical, nrc, status, order, st, probe);
+}
+
+cudaError_t launch_cache_paths(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
+                               uint32_t max_depth, const NrcShadeArgs& nrc, DeviceStatus* status, int order,
+                               cudaStream_t st)
+{
+    const cudaError_t e = cudaMemsetAsync(nrc.count, 0, nrc.passes * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    return launch_paths(sc, b, cam, seed, max_depth, true, nrc, status, order, st, nullptr);
+}
+
+cudaError_t launch_cache_answers(PathBatch& b, const NrcShadeArgs& na, uint32_t pass, cudaStream_t st)
+{
+    return nrc::launch_infer(na.geo, na.table, na.weights, na.queries + 4 * (size_t)pass * na.capacity, na.capacity,
+                             nullptr, b.thr, b.pay, na.err, st, na.count + pass, na.infer_groups, na.wait);
+}
+
+cudaError_t launch_accumulate(PathBatch& b, uint32_t spb, uint32_t max_samples, float max_variance, bool physical,
+                              DeviceStatus* status, cudaStream_t st)
+{
+    b.sample_tally = &status->rays[3];
+    accumulate_kernel<<<grid_for(accumulate_kernel, b.npix, kRenderThreads), kRenderThreads, 0, st>>>(
+        b, spb, max_samples, max_variance, physical);
     return cudaGetLastError();
 }
 
 cudaError_t launch_render_batch(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
                                 uint32_t spb, uint32_t max_depth, uint32_t max_samples, float max_variance,
                                 int estimator, DeviceStatus* status, int order, cudaStream_t st,
-                                const NrcShadeArgs* nrc, const RenderProbe* probe)
+                                const RenderProbe* probe)
 {
-    b.sample_tally = &status->rays[3];
     const bool physical = estimator != PICO_ESTIMATOR_REFERENCE;
     NrcShadeArgs off{};
     off.mode = kNrcOff;
-    const NrcShadeArgs& na = nrc ? *nrc : off;
-    cudaError_t e = cudaMemsetAsync(b.depths, 0, kDepthRing * sizeof(DepthQueues), st);
-    if (e == cudaSuccess && na.mode != kNrcOff) e = cudaMemsetAsync(na.count, 0, sizeof(uint32_t), st);
+    const cudaError_t e = launch_paths(sc, b, cam, seed, max_depth, physical, off, status, order, st, probe);
     if (e != cudaSuccess) return e;
-    raygen_kernel<<<grid_for(raygen_kernel, b.n, kRenderThreads), kRenderThreads, 0, st>>>(b, cam, seed, physical);
-    e = run_depth_loop(sc, b, max_depth, physical, na, status, order, st, probe);
-    if (e != cudaSuccess) return e;
-    if (na.mode == kNrcTerminate) {
-        e = nrc::launch_infer(na.geo, na.table, na.weights, na.queries, na.capacity, nullptr, b.thr, b.pay, na.err, st,
-                              na.count, na.infer_groups, na.wait);
-        if (e != cudaSuccess) return e;
-    }
-    accumulate_kernel<<<grid_for(accumulate_kernel, b.npix, kRenderThreads), kRenderThreads, 0, st>>>(b, spb, max_samples, max_variance,
-                                                                                    physical);
-    return cudaGetLastError();
+    return launch_accumulate(b, spb, max_samples, max_variance, physical, status, st);
 }
 
 cudaError_t launch_plan_init(RoundPlan* plan, uint32_t npix, cudaStream_t st)

@@ -124,11 +124,13 @@ struct RenderProbe {
 enum NrcMode { kNrcOff = 0, kNrcRecord = 1, kNrcTerminate = 2 };
 struct NrcShadeArgs {
     int mode;
-    uint32_t capacity;        // entries of queries / rec_tp
+    uint32_t passes;          // passes traced together, pass p on paths [p * pass_paths, (p + 1) * pass_paths)
+    uint32_t pass_paths;
+    uint32_t capacity;        // entries of queries / rec_tp per pass
     uint32_t bounces;         // kNrcTerminate: bounces before the cache answers (one more behind a glossy vertex)
-    float4* queries;          // 4 float4 per entry (pico_nrc_query)
+    float4* queries;          // 4 float4 per entry (pico_nrc_query); pass p's from entry p * capacity on
     float4* rec_tp;           // kNrcRecord: 2 float4 per entry
-    uint32_t* count;          // entries appended
+    uint32_t* count;          // entries appended, per pass
     float* prev_rough;        // kNrcTerminate: per path, roughness of its previous vertex
     // the cache the terminating paths query
     nrc::GridGeometry geo;
@@ -142,7 +144,7 @@ struct NrcShadeArgs {
 cudaError_t launch_render_batch(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
                                 uint32_t spb, uint32_t max_depth, uint32_t max_samples, float max_variance,
                                 int estimator, DeviceStatus* status, int order, cudaStream_t st,
-                                const NrcShadeArgs* nrc = nullptr, const RenderProbe* probe = nullptr);
+                                const RenderProbe* probe = nullptr);
 // Exit-aware rounds: plan_init lists npix pixels for the first round; plan_round
 // sets the next round from the pixels the compaction kept: samples per pixel
 // min(max_samples - scheduled, max_paths / pixels, cap), at most first_cap in the
@@ -157,14 +159,22 @@ cudaError_t launch_compact_pixels(RoundPlan* plan, const uint32_t* in, const uin
 // tile order (tile_pixel), done where count >= max_samples, nothing taken yet.
 cudaError_t launch_prepare_image(const uint32_t* count, uint32_t W, uint32_t H, uint32_t max_samples,
                                  uint32_t* pix_list, uint32_t* done, uint32_t* taken, cudaStream_t st);
-// The radiance cache's training paths of one sample pass: n full-depth physical
-// paths from pseudo-random pixels of the W x H image (path slots 0 .. n-1 of b),
-// recording every shaded vertex (kNrcRecord), then the records' targets
-// (4 floats each) in `targets`.
+// The radiance cache's training paths of nrc.passes sample passes: nrc.pass_paths
+// full-depth physical paths each, from pseudo-random pixels of the W x H image (path
+// slots of b from 0 on; pass p draws with frame + p), recording every shaded vertex
+// (kNrcRecord), then the records' targets (4 floats each) in `targets`.
 cudaError_t launch_training_paths(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
-                                  uint32_t frame, uint32_t n, uint32_t W, uint32_t H, uint32_t max_depth,
-                                  const NrcShadeArgs& nrc, float4* targets, DeviceStatus* status, int order,
-                                  cudaStream_t st);
+                                  uint32_t frame, uint32_t W, uint32_t H, uint32_t max_depth, const NrcShadeArgs& nrc,
+                                  float4* targets, DeviceStatus* status, int order, cudaStream_t st);
+// One sample per pixel of b and pass of nrc (kNrcTerminate), each path up to the vertex
+// that it ends at in the cache; launch_cache_answers adds pass p's answers, and
+// launch_accumulate then takes the samples of all passes.
+cudaError_t launch_cache_paths(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
+                               uint32_t max_depth, const NrcShadeArgs& nrc, DeviceStatus* status, int order,
+                               cudaStream_t st);
+cudaError_t launch_cache_answers(PathBatch& b, const NrcShadeArgs& nrc, uint32_t pass, cudaStream_t st);
+cudaError_t launch_accumulate(PathBatch& b, uint32_t spb, uint32_t max_samples, float max_variance, bool physical,
+                              DeviceStatus* status, cudaStream_t st);
 // Writes the device's global nanosecond timer to *dst when the stream reaches it.
 cudaError_t launch_stamp(unsigned long long* dst, cudaStream_t st);
 cudaError_t launch_gbuffer(const SceneView& sc, const CameraView& cam, uint32_t W, uint32_t H, float* normals,
