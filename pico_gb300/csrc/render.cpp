@@ -173,12 +173,12 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
     const uint32_t ntrain = std::min<uint32_t>(c->cfg.train_paths, path_limit(ctx));
     const uint32_t max_depth = cfg->max_ray_depth;
     const uint32_t passes = c->cfg.warmup_frames + cfg->max_samples;
-    // passes of a group: as many as 2^24 paths hold, one when the image takes several chunks, fewer where the device's
-    // memory has no room for their state
-    const uint32_t room = std::min(path_limit(ctx), 1u << 24);
-    uint32_t group = std::max(1u, std::min({kCancelSamplesPerBatch, passes,
-                                            chunk_pix < nactive ? 1u : room / std::max({chunk_pix, ntrain, 1u})}));
     const uint32_t rec_cap = (uint32_t)std::min<uint64_t>((uint64_t)ntrain * std::max(max_depth, 1u), 0xffffffffu);
+    // passes of a group: as many as 2^24 paths and 2^24 training records (112 bytes each, max_depth of them a training
+    // path) hold, one when the image takes several chunks, fewer where the device's memory has no room for their state
+    const uint32_t room = std::min(path_limit(ctx), 1u << 24);
+    uint32_t group = std::max(1u, std::min({kCancelSamplesPerBatch, passes, (1u << 24) / std::max(rec_cap, 1u),
+                                            chunk_pix < nactive ? 1u : room / std::max({chunk_pix, ntrain, 1u})}));
     cudaError_t e = cudaSuccess;
     for (;; group /= 2) {
         const size_t slots = (size_t)group * std::max<size_t>(chunk_pix, ntrain);
