@@ -6,21 +6,24 @@
 // blend needs the maximum luminance and the min / max |position| over every
 // pixel some tap of the tile reads.  That set is rows x columns, each a union of
 // five shifted copies of the tile's range, clamped.  The positions are the same
-// at every level, so two launches first reduce all five levels' |position|
-// ranges, separably (per image row over each tile column's footprint columns,
-// then per tile over its footprint rows), reading the positions once; then each
-// level runs two kernels:
+// at every level, so all five levels' |position| ranges are reduced first,
+// separably (per image row over each tile column's footprint columns, then per
+// tile over its footprint rows), reading the positions once, beside the packing
+// of the inputs into records (prepare, tile_range).  Then each level runs:
 //
-//   stats  the maximum luminance of the level's input colour over the tile's
-//          footprint (four CTAs per tile, each a quarter of the footprint rows),
-//          walking the distinct members once instead of 25 taps per pixel.
-//          max / min are exact, so the order is free, and the selects keep
-//          std::max / std::min's NaN behaviour.
-//   blend  one thread per pixel: 25 taps, weights
+//   white  the maximum luminance of the level's input colour over each tile's
+//          footprint: from the luminance cells that the blend before filled, or
+//          (first level; images whose last tile is narrower than the spacing)
+//          from the colours (stats: four CTAs per tile, each a quarter of the
+//          footprint rows).  max / min are exact, so the order is free, and the
+//          selects keep std::max / std::min's NaN behaviour.
+//   blend  25 taps a pixel, weights
 //          w = k[u] * min(exp(-|dn|^2/0.25),1) * min(exp(-|dp|^2/range^2),1)
 //                   * min(exp(-|dalbedo|^2/white^2),1),
 //          out = sum(w * c) / sum(w), evaluated with one exponential per tap
 //          (see the kernel).
+//
+// 1920 x 1080: 621 us before the records, cells and tiles below, 468 now.
 //
 // The statistics are exact; the blend agrees with the reference's arithmetic to
 // about 1e-6 relative and keeps its NaN pattern.
@@ -31,13 +34,20 @@
 
 namespace pico {
 
-__constant__ float kAtrousWeights[25] = {
-    0.00292f, 0.01306f, 0.02154f, 0.01306f, 0.00292f,
-    0.01306f, 0.05855f, 0.09653f, 0.05855f, 0.01306f,
-    0.02154f, 0.09653f, 0.15915f, 0.09653f, 0.02154f,
-    0.01306f, 0.05855f, 0.09563f, 0.05855f, 0.01306f,
-    0.00292f, 0.01306f, 0.02154f, 0.01306f, 0.00292f};
+// Base-2 logarithms of the 5x5 table:
+//   0.00292, 0.01306, 0.02154, 0.01306, 0.00292
+//   0.01306, 0.05855, 0.09653, 0.05855, 0.01306
+//   0.02154, 0.09653, 0.15915, 0.09653, 0.02154
+//   0.01306, 0.05855, 0.09563, 0.05855, 0.01306
+//   0.00292, 0.01306, 0.02154, 0.01306, 0.00292
+__constant__ float kAtrousLog2[25] = {
+    -8.41981602f, -6.25870132f, -5.53683805f, -6.25870132f, -8.41981602f,
+    -6.25870132f, -4.09418678f, -3.37287879f, -4.09418678f, -6.25870132f,
+    -5.53683805f, -3.37287879f, -2.65154099f, -3.37287879f, -5.53683805f,
+    -6.25870132f, -4.09418678f, -3.38639283f, -4.09418678f, -6.25870132f,
+    -8.41981602f, -6.25870132f, -5.53683805f, -6.25870132f, -8.41981602f};
 
+constexpr float kLog2e = 1.44269504f;
 constexpr int kTile = 64;
 constexpr int kStatsThreads = 256;
 constexpr int kStatsSplit = 4;   // CTAs per tile; each reduces every fourth footprint row group
@@ -82,10 +92,11 @@ __device__ __forceinline__ float luminance(float r, float g, float b)
     return add(add(mul(r, 0.2126f), mul(g, 0.587f)), mul(b, 0.114f));
 }
 
-// Maximum luminance over this CTA's quarter of a tile's footprint rows (a partial
-// record per CTA; tile_stats combines the four).
-__global__ void __launch_bounds__(kStatsThreads) atrous_stats_kernel(const float* __restrict__ pix, uint32_t W,
-                                                                      uint32_t H, int s, float* __restrict__ parts)
+// Maximum luminance over this CTA's quarter of a tile's footprint rows, into the tile's
+// white point (cleared before; non-negative floats order like their bits).
+__global__ void __launch_bounds__(kStatsThreads) atrous_stats_kernel(const float* __restrict__ pix, int stride,
+                                                                     uint32_t W, uint32_t H, int s,
+                                                                     uint32_t* __restrict__ white_bits)
 {
     const int tiles_x = (int)((W + kTile - 1) / kTile);
     const int tile = (int)(blockIdx.x / kStatsSplit), part = (int)(blockIdx.x % kStatsSplit);
@@ -109,7 +120,8 @@ __global__ void __launch_bounds__(kStatsThreads) atrous_stats_kernel(const float
         const size_t rb = (size_t)rows[r] * W;
         for (int c = lane; c < ncols; c += 32) {
             const size_t f = rb + (size_t)cols[c];
-            const float l = luminance(__ldg(pix + 3 * f), __ldg(pix + 3 * f + 1), __ldg(pix + 3 * f + 2));
+            const float* p = pix + stride * f;
+            const float l = luminance(__ldg(p), __ldg(p + 1), __ldg(p + 2));
             white = (white < l) ? l : white;
         }
     }
@@ -122,7 +134,7 @@ __global__ void __launch_bounds__(kStatsThreads) atrous_stats_kernel(const float
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < kWarps; ++w) white = (white < sw[w]) ? sw[w] : white;
-        parts[blockIdx.x] = white;
+        atomicMax(white_bits + tile, __float_as_uint(white));
     }
 }
 
@@ -148,13 +160,14 @@ __device__ __forceinline__ bool tapped(int c, int a, int b, int s, int n)
     return in;
 }
 
-__global__ void __launch_bounds__(32 * kRowWarps) atrous_row_range_kernel(const float* __restrict__ pos, uint32_t W,
-                                                                        uint32_t H, float2* __restrict__ rrow)
+// Rows kRowWarps * block .. of the image's (row, tile column) pairs.
+__device__ __forceinline__ void row_range(uint32_t block, const float* __restrict__ pos, uint32_t W, uint32_t H,
+                                          float2* __restrict__ rrow)
 {
     using namespace ex;
     const int tiles_x = (int)((W + kTile - 1) / kTile);
     const int lane = threadIdx.x & 31;
-    const long long task = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    const long long task = (long long)block * kRowWarps + (threadIdx.x >> 5);
     if (task >= (long long)H * tiles_x) return;   // the whole warp leaves together
     const int y = (int)(task / tiles_x), tx = (int)(task % tiles_x);
     const int x0 = tx * kTile, x1 = min(x0 + kTile, (int)W) - 1;
@@ -195,18 +208,15 @@ __global__ void __launch_bounds__(32 * kRowWarps) atrous_row_range_kernel(const 
                 maxd = (maxd < len[k]) ? len[k] : maxd;
             }
         }
-        for (int off = 16; off > 0; off >>= 1) {
-            const float a2 = __shfl_down_sync(0xffffffffu, mind, off);
-            const float b2 = __shfl_down_sync(0xffffffffu, maxd, off);
-            mind = (a2 < mind) ? a2 : mind;
-            maxd = (maxd < b2) ? b2 : maxd;
-        }
+        // neither is a NaN, and lengths order like their bits (the empty maximum, -inf, as a negative integer)
+        mind = __int_as_float(__reduce_min_sync(0xffffffffu, __float_as_int(mind)));
+        maxd = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(maxd)));
         if (lane == 0) rrow[((size_t)level * H + y) * tiles_x + tx] = make_float2(mind, maxd);
     }
 }
 
 __global__ void __launch_bounds__(32 * 5) atrous_tile_range_kernel(const float2* __restrict__ rrow, uint32_t W,
-                                                                   uint32_t H, float2* __restrict__ range)
+                                                                   uint32_t H, float* __restrict__ pos_scale)
 {
     const int tiles_x = (int)((W + kTile - 1) / kTile);
     const int tiles = tiles_x * (int)((H + kTile - 1) / kTile);
@@ -229,223 +239,260 @@ __global__ void __launch_bounds__(32 * 5) atrous_tile_range_kernel(const float2*
         mind = (a2 < mind) ? a2 : mind;
         maxd = (maxd < b2) ? b2 : maxd;
     }
-    if (lane == 0) range[level * tiles + tile] = make_float2(mind, maxd);
-}
-
-// A tile's white point (from its kStatsSplit partial records) and |position| range.
-__device__ __forceinline__ float2 tile_stats(const float* __restrict__ parts, const float2* __restrict__ range,
-                                             int tile)
-{
-    float w = parts[tile * kStatsSplit];
-#pragma unroll
-    for (int k = 1; k < kStatsSplit; ++k) {
-        const float p = parts[tile * kStatsSplit + k];
-        w = (w < p) ? p : w;
+    if (lane == 0) {
+        const float d = __fsub_rn(maxd, mind);
+        pos_scale[level * tiles + tile] = -kLog2e * __frcp_rn(__fmul_rn(d, d));   // -inf for a zero range
     }
-    const float2 r = range[tile];
-    return make_float2(w, __fsub_rn(r.y, r.x));
 }
 
-// One thread per pixel, 25 taps.  The reference's weight
+// The blend reads its taps as packed records of 48 bytes a pixel: (normal x, position x, normal y, position y),
+// (normal z, position z, albedo x, albedo y) side by side, written once, and (albedo z, colour) in an array of its own,
+// written by each level for the next.  A tap is three 128-bit loads instead of twelve of 4 bytes, and the normal and
+// the position advance in pairs through packed float operations.
+__device__ __forceinline__ void pack(size_t i, const float* __restrict__ pix, const float* __restrict__ nrm,
+                                     const float* __restrict__ pos, const float* __restrict__ dif, size_t npx,
+                                     float4* __restrict__ ab, float4* __restrict__ c)
+{
+    if (i >= npx) return;
+    const float *n = nrm + 3 * i, *p = pos + 3 * i, *d = dif + 3 * i, *x = pix + 3 * i;
+    ab[2 * i] = make_float4(__ldg(n), __ldg(p), __ldg(n + 1), __ldg(p + 1));
+    ab[2 * i + 1] = make_float4(__ldg(n + 2), __ldg(p + 2), __ldg(d), __ldg(d + 1));
+    c[i] = make_float4(__ldg(d + 2), __ldg(x), __ldg(x + 1), __ldg(x + 2));
+}
+
+// Both of these and the clearing of a call's white points and cells in one launch: the row ranges are bound by
+// instruction issue (21 us alone) and the packing by memory (31 us), so every third block takes rows and the others
+// pack, and they share the SMs.
+constexpr int kPrepareThreads = 32 * kRowWarps;
+__global__ void __launch_bounds__(kPrepareThreads) atrous_prepare_kernel(
+    const float* __restrict__ pix, const float* __restrict__ nrm, const float* __restrict__ pos,
+    const float* __restrict__ dif, uint32_t W, uint32_t H, float4* __restrict__ ab, float4* __restrict__ c,
+    float2* __restrict__ rrow, uint32_t* __restrict__ white, size_t nwhite, uint32_t* __restrict__ cells, size_t ncells)
+{
+    if (blockIdx.x % 3 == 0) {
+        row_range(blockIdx.x / 3, pos, W, H, rrow);
+        return;
+    }
+    const size_t i = (size_t)(blockIdx.x - blockIdx.x / 3 - 1) * kPrepareThreads + threadIdx.x;
+    if (i < nwhite) white[i] = 0;
+    if (i < ncells) cells[i] = 0;
+    pack(i, pix, nrm, pos, dif, (size_t)W * H, ab, c);
+}
+
+// The white points of a level from the cells that the level before it filled: cells of 2 s x 2 s pixels, each with
+// its largest luminance (from 0).  A tile's footprint at spacing s is the whole rectangle from its first column and
+// row less 2 s to its last plus 2 s, clamped (whole_footprints), and all its sides lie on cell borders or on the
+// image's.  One warp per tile.
+__global__ void __launch_bounds__(128) atrous_white_kernel(const uint32_t* __restrict__ cells, uint32_t W, uint32_t H,
+                                                           int s, float* __restrict__ white)
+{
+    const uint32_t tiles_x = (W + kTile - 1) / kTile, tiles = tiles_x * ((H + kTile - 1) / kTile);
+    const uint32_t tile = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (tile >= tiles) return;   // the whole warp leaves together
+    const int x0 = (int)(tile % tiles_x) * kTile, y0 = (int)(tile / tiles_x) * kTile, c = 2 * s;
+    const int cx0 = max(x0 - c, 0) / c, cx1 = min(x0 + kTile - 1 + c, (int)W - 1) / c;
+    const int cy0 = max(y0 - c, 0) / c, cy1 = min(y0 + kTile - 1 + c, (int)H - 1) / c;
+    const int nx = cx1 - cx0 + 1, n = nx * (cy1 - cy0 + 1);
+    const size_t pitch = (W + c - 1) / c;
+    uint32_t m = 0;   // non-negative floats order like their bits
+    for (int k = (int)lane; k < n; k += 32) m = max(m, __ldg(cells + (size_t)(cy0 + k / nx) * pitch + (cx0 + k % nx)));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) white[tile] = __uint_as_float(m);
+}
+
+// Whether every tile's footprint at spacing s is one rectangle: its taps' ranges overlap when the tile is at least s
+// wide and high, which only the last column and row of tiles may miss.
+static bool whole_footprints(uint32_t W, uint32_t H, int s)
+{
+    auto whole = [s](uint32_t n) { const uint32_t last = n % kTile; return last == 0 || last >= (uint32_t)s; };
+    return whole(W) && whole(H);
+}
+
+// The blend: 25 taps per pixel.  The reference's weight
 //   k[u] * min(exp(-|dn|^2/0.25),1) * min(exp(-|dp|^2/range^2),1) * min(exp(-|da|^2/white^2),1)
-// is evaluated as k[u] * exp(-(4|dn|^2 + |dp|^2 * (1/range^2) + |da|^2 * (1/white^2))): the
-// arguments are never positive, so the min(., 1) clamps only pass NaN through, and a sum
-// of -inf / NaN terms gives the same 0 / NaN as the product of exponentials.  One fast
-// exponential per tap instead of three exact ones and three divides; the result stays
-// within 1e-5 relative of the exact evaluation (the weights enter a normalised sum in
-// which the centre tap, k = 0.159, always has exponent 0).
-template <typename Idx>
-__global__ void __launch_bounds__(256) atrous_blend_kernel(const float* __restrict__ src,
-                                                           const float* __restrict__ nrm,
-                                                           const float* __restrict__ pos,
-                                                           const float* __restrict__ dif, uint32_t W, uint32_t H,
-                                                           int s, const float* __restrict__ stats,
-                                                           const float2* __restrict__ range, float* __restrict__ dst)
+// is evaluated as 2^(log2 k[u] - |dn|^2 4 log2 e - |dp|^2 log2 e / range^2 - |da|^2 log2 e / white^2): the arguments
+// of the exponentials are never positive, so the min(., 1) clamps only pass NaN through, and a sum of -inf / NaN
+// terms gives the same 0 / NaN as their product.  One hardware exponential per tap; the result stays within 1e-5
+// relative of the exact evaluation (the weights enter a normalised sum in which the centre tap, k = 0.159, always
+// has exponent 0).
+//
+// At spacing s every tap of a pixel lands on the pixel's own sub-lattice (x mod s, y mod s), so a CTA takes a
+// kLatX x kLatY tile of one sub-lattice at every spacing; the (kLatX + 4) x (kLatY + 4) lattice points its taps read
+// (coordinates clamped exactly as the taps clamp them) are copied to shared memory once, asynchronously and past L1.
+// Each thread blends two neighbouring columns, whose taps overlap, and reads each record once for both; the records of
+// a footprint row are split into even and odd columns so that a warp's loads hit consecutive records.
+//
+// Measured at 1920 x 1080 (start 92-98 us a level with its own tile kernel for spacings 1-4 and a direct one above):
+// 72-79 us a level at 60 % of the issue slots, 62 % of the shared-memory wavefronts and half of the FP32 pipe (whose
+// 36 us a level are the floor), 24 warps per SM waiting on shared-memory latency between.  Whole call: copies through
+// registers 595 us against 534 asynchronous; scalar differences 30 us more than packed ones; two rows per thread
+// (fewer reads, 20 warps) 528 against 509, three 605 against 534; 7 or 8 CTAs per SM (72 or 64 registers) 515 and 528;
+// tiles of 64 x 8, 32 x 16, 16 x 16 and 16 x 8 points 5, 5, 3 and 1 % slower.
+//
+// With `cells`, the pixels' luminances go to the next level's white points: the largest of each cell of 4 s x 4 s
+// pixels, 4 x 4 points of every sub-lattice.  A level's white points take 4-6 us from cells, 13 from the colours.
+__device__ __forceinline__ void copy16(float4* to, const float4* from)
 {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= W) return;
-    const int tiles_x = (int)((W + kTile - 1) / kTile);
-    const float2 st = tile_stats(stats, range, (int)((y / kTile) * tiles_x + x / kTile));
-    const float ip = __frcp_rn(__fmul_rn(st.y, st.y));   // 1 / range^2 (inf for a zero range)
-    const float iw = __frcp_rn(__fmul_rn(st.x, st.x));   // 1 / white^2
-    const Idx c = ((Idx)y * W + x) * 3;
-    const float ncx = nrm[c], ncy = nrm[c + 1], ncz = nrm[c + 2];
-    const float pcx = pos[c], pcy = pos[c + 1], pcz = pos[c + 2];
-    const float dcx = dif[c], dcy = dif[c + 1], dcz = dif[c + 2];
-    Idx col[5], row[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        col[k] = (Idx)clampi((int)x + (k - 2) * s, 0, (int)W - 1) * 3;
-        row[k] = (Idx)clampi((int)y + (k - 2) * s, 0, (int)H - 1) * W * 3;
-    }
-    float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f, wsum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 5; ++j) {
-#pragma unroll
-        for (int i = 0; i < 5; ++i) {
-            const Idx f = row[j] + col[i];
-            const float nx = ncx - __ldg(nrm + f), ny = ncy - __ldg(nrm + f + 1), nz = ncz - __ldg(nrm + f + 2);
-            const float px = pcx - __ldg(pos + f), py = pcy - __ldg(pos + f + 1), pz = pcz - __ldg(pos + f + 2);
-            const float ax = dcx - __ldg(dif + f), ay = dcy - __ldg(dif + f + 1), az = dcz - __ldg(dif + f + 2);
-            const float dn = nx * nx + ny * ny + nz * nz;
-            const float dp = px * px + py * py + pz * pz;
-            const float da = ax * ax + ay * ay + az * az;
-            const float w = kAtrousWeights[j * 5 + i] * __expf(-(4.0f * dn + dp * ip + da * iw));
-            r0 += __ldg(src + f) * w;
-            r1 += __ldg(src + f + 1) * w;
-            r2 += __ldg(src + f + 2) * w;
-            wsum += w;
-        }
-    }
-    dst[c] = __fdiv_rn(r0, wsum);
-    dst[c + 1] = __fdiv_rn(r1, wsum);
-    dst[c + 2] = __fdiv_rn(r2, wsum);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+                 : "memory");
 }
 
-// The same blend with its taps staged in shared memory, for small spacings.  At
-// spacing s every tap of a pixel lands on the pixel's own sub-lattice (x mod s,
-// y mod s), so a CTA takes a kLatX x kLatY tile of one sub-lattice; the
-// (kLatX + 4) x (kLatY + 4) lattice points its taps read (coordinates clamped
-// exactly as the taps clamp them) are staged once as 48-byte records (normal,
-// position, albedo, colour) and read back with 128-bit loads.  Each thread blends
-// two horizontally adjacent lattice pixels, which share four of their five tap
-// columns; the records of a footprint row are split into even and odd columns so
-// that a warp's loads hit consecutive records.  The arithmetic per tap is the
-// direct kernel's above, so the two kernels give identical results.
-constexpr int kLatX = 64, kLatY = 8, kBlendThreads = (kLatX / 2) * kLatY;
+constexpr int kLatX = 32, kLatY = 8, kBlendThreads = kLatX / 2 * kLatY;
 constexpr int kFootX = kLatX + 4, kHalfX = kFootX / 2, kFootY = kLatY + 4;
 
-__device__ __forceinline__ void blend_tap(const float4 t0, const float4 t1, const float4 t2, float k, const float* c,
-                                          float ip, float iw, float* acc)
-{
-    const float nx = c[0] - t0.x, ny = c[1] - t0.y, nz = c[2] - t0.z;
-    const float px = c[3] - t0.w, py = c[4] - t1.x, pz = c[5] - t1.y;
-    const float ax = c[6] - t1.z, ay = c[7] - t1.w, az = c[8] - t2.x;
-    const float dn = nx * nx + ny * ny + nz * nz;
-    const float dp = px * px + py * py + pz * pz;
-    const float da = ax * ax + ay * ay + az * az;
-    const float w = k * __expf(-(4.0f * dn + dp * ip + da * iw));
-    acc[0] += t2.y * w;
-    acc[1] += t2.z * w;
-    acc[2] += t2.w * w;
-    acc[3] += w;
-}
-
-template <typename Idx>
-__global__ void __launch_bounds__(kBlendThreads) atrous_blend_tiled_kernel(
-    const float* __restrict__ src, const float* __restrict__ nrm, const float* __restrict__ pos,
-    const float* __restrict__ dif, uint32_t W, uint32_t H, int s, const float* __restrict__ stats,
-    const float2* __restrict__ range, float* __restrict__ dst)
+__global__ void __launch_bounds__(kBlendThreads, 6) atrous_blend_kernel(
+    const float4* __restrict__ rab, const float4* __restrict__ rc, uint32_t W, uint32_t H, int shift, uint32_t cols,
+    const float* __restrict__ white, const float* __restrict__ pos_scale, float4* __restrict__ dst,
+    uint32_t* __restrict__ cells, uint32_t cell_pitch)
 {
     __shared__ float4 rec[kFootY * kFootX * 3];   // [row][column parity][column / 2] records
-    const int rx = (int)(blockIdx.x % (uint32_t)s), tx = (int)(blockIdx.x / (uint32_t)s);
-    const int ry = (int)(blockIdx.y % (uint32_t)s), ty = (int)(blockIdx.y / (uint32_t)s);
+    const int s = 1 << shift;
+    const int by = (int)(blockIdx.x / cols), bx = (int)(blockIdx.x - (uint32_t)by * cols);
+    const int rx = bx & (s - 1), tx = bx >> shift, ry = by & (s - 1), ty = by >> shift;
     const int lx0 = tx * kLatX - 2, ly0 = ty * kLatY - 2;   // lattice coordinate of footprint entry (0, 0)
-    for (int e = threadIdx.x; e < kFootX * kFootY; e += blockDim.x) {
-        const int ex = e % kFootX, ey = e / kFootX;
+    int ex = (int)threadIdx.x % kFootX, ey = (int)threadIdx.x / kFootX;
+    for (int e = (int)threadIdx.x; e < kFootX * kFootY; e += kBlendThreads) {
         const int x = clampi(rx + (lx0 + ex) * s, 0, (int)W - 1);
         const int y = clampi(ry + (ly0 + ey) * s, 0, (int)H - 1);
-        const Idx f = ((Idx)y * W + (Idx)x) * 3;
-        const int slot = 3 * ((ey * 2 + (ex & 1)) * kHalfX + (ex >> 1));
-        rec[slot] = make_float4(__ldg(nrm + f), __ldg(nrm + f + 1), __ldg(nrm + f + 2), __ldg(pos + f));
-        rec[slot + 1] = make_float4(__ldg(pos + f + 1), __ldg(pos + f + 2), __ldg(dif + f), __ldg(dif + f + 1));
-        rec[slot + 2] = make_float4(__ldg(dif + f + 2), __ldg(src + f), __ldg(src + f + 1), __ldg(src + f + 2));
+        const size_t f = (size_t)y * W + (size_t)x;
+        float4* slot = rec + 3 * ((ey * 2 + (ex & 1)) * kHalfX + (ex >> 1));
+        copy16(slot, rab + 2 * f);
+        copy16(slot + 1, rab + 2 * f + 1);
+        copy16(slot + 2, rc + f);
+        ex += kBlendThreads % kFootX;
+        ey += kBlendThreads / kFootX;
+        if (ex >= kFootX) { ex -= kFootX; ++ey; }
     }
+    const int h = (int)(threadIdx.x % (kLatX / 2)), row = (int)(threadIdx.x / (kLatX / 2));
+    const uint32_t tiles_x = (W + kTile - 1) / kTile;
+    const int x0 = rx + (tx * kLatX + 2 * h) * s, y0 = ry + (ty * kLatY + row) * s;   // the thread's first pixel
+    float ctr[2][9], acc[2][4], ip[2], iw[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const uint32_t x = min((uint32_t)(x0 + k * s), W - 1), y = min((uint32_t)y0, H - 1);
+        const size_t tile = (size_t)(y / kTile) * tiles_x + x / kTile;
+        const float w = __ldg(white + tile);
+        ip[k] = __ldg(pos_scale + tile);                // -log2 e / range^2
+        iw[k] = -kLog2e * __frcp_rn(__fmul_rn(w, w));   // -log2 e / white^2
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[k][u] = 0.0f;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const int h = (int)(threadIdx.x % (kLatX / 2)), b = (int)(threadIdx.x / (kLatX / 2));
-    const int a = 2 * h;                                     // this thread's lattice pixels: a and a + 1
-    const int y = ry + (ty * kLatY + b) * s;
-    const int x0 = rx + (tx * kLatX + a) * s, x1 = x0 + s;
-    if (y >= (int)H || x0 >= (int)W) return;
-    const int tiles_x = (int)((W + kTile - 1) / kTile);
-    const int x1c = x1 < (int)W ? x1 : x0;
-    const float2 st0 = tile_stats(stats, range, (y / kTile) * tiles_x + x0 / kTile);
-    const float2 st1 = tile_stats(stats, range, (y / kTile) * tiles_x + x1c / kTile);
-    const float ip0 = __frcp_rn(__fmul_rn(st0.y, st0.y)), iw0 = __frcp_rn(__fmul_rn(st0.x, st0.x));
-    const float ip1 = __frcp_rn(__fmul_rn(st1.y, st1.y)), iw1 = __frcp_rn(__fmul_rn(st1.x, st1.x));
-    float c0[9], c1[9];
-    {
-        const int r0 = 3 * (((b + 2) * 2 + 0) * kHalfX + h + 1);   // column a + 2 (even)
-        const int r1 = 3 * (((b + 2) * 2 + 1) * kHalfX + h + 1);   // column a + 3 (odd)
-        const float4 p0 = rec[r0], p1 = rec[r0 + 1], p2 = rec[r0 + 2];
-        const float4 q0 = rec[r1], q1 = rec[r1 + 1], q2 = rec[r1 + 2];
-        c0[0] = p0.x; c0[1] = p0.y; c0[2] = p0.z; c0[3] = p0.w; c0[4] = p1.x; c0[5] = p1.y;
-        c0[6] = p1.z; c0[7] = p1.w; c0[8] = p2.x;
-        c1[0] = q0.x; c1[1] = q0.y; c1[2] = q0.z; c1[3] = q0.w; c1[4] = q1.x; c1[5] = q1.y;
-        c1[6] = q1.z; c1[7] = q1.w; c1[8] = q2.x;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float4* c = rec + 3 * (((row + 2) * 2 + k) * kHalfX + h + 1);   // footprint column 2 h + 2 + k
+        const float4 a = c[0], b = c[1];
+        float* p = ctr[k];
+        p[0] = -a.x; p[1] = -a.y; p[2] = -a.z; p[3] = -a.w; p[4] = -b.x; p[5] = -b.y; p[6] = -b.z; p[7] = -b.w;
+        p[8] = -c[2].x;
     }
-    float acc0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, acc1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {   // footprint column a + q
-            const int r = 3 * (((b + j) * 2 + (q & 1)) * kHalfX + h + (q >> 1));
-            const float4 t0 = rec[r], t1 = rec[r + 1], t2 = rec[r + 2];
-            if (q <= 4) blend_tap(t0, t1, t2, kAtrousWeights[j * 5 + q], c0, ip0, iw0, acc0);
-            if (q >= 1) blend_tap(t0, t1, t2, kAtrousWeights[j * 5 + q - 1], c1, ip1, iw1, acc1);
+        for (int q = 0; q < 6; ++q) {   // footprint column 2 h + q: tap column q - k of pixel k
+            const float4* t = rec + 3 * (((row + j) * 2 + (q & 1)) * kHalfX + h + (q >> 1));
+            const float4 a = t[0], b = t[1], c = t[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int i = q - k;
+                if (i < 0 || i > 4) continue;
+                const float* p = ctr[k];
+                const float2 x = __fadd2_rn(make_float2(a.x, a.y), make_float2(p[0], p[1]));
+                const float2 y = __fadd2_rn(make_float2(a.z, a.w), make_float2(p[2], p[3]));
+                const float2 z = __fadd2_rn(make_float2(b.x, b.y), make_float2(p[4], p[5]));
+                const float2 v = __fadd2_rn(make_float2(b.z, b.w), make_float2(p[6], p[7]));
+                const float az = p[8] + c.x;
+                const float2 np = __ffma2_rn(z, z, __ffma2_rn(y, y, __fmul2_rn(x, x)));   // |dn|^2, |dp|^2
+                const float2 vv = __fmul2_rn(v, v);
+                const float da = fmaf(az, az, vv.x) + vv.y;
+                const float e = fmaf(da, iw[k], fmaf(np.y, ip[k], fmaf(np.x, -4.0f * kLog2e, kAtrousLog2[j * 5 + i])));
+                float w;
+                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(e));
+                acc[k][0] = fmaf(c.y, w, acc[k][0]);
+                acc[k][1] = fmaf(c.z, w, acc[k][1]);
+                acc[k][2] = fmaf(c.w, w, acc[k][2]);
+                acc[k][3] += w;
+            }
         }
     }
-    const Idx o0 = ((Idx)y * W + (Idx)x0) * 3;
-    dst[o0] = __fdiv_rn(acc0[0], acc0[3]);
-    dst[o0 + 1] = __fdiv_rn(acc0[1], acc0[3]);
-    dst[o0 + 2] = __fdiv_rn(acc0[2], acc0[3]);
-    if (x1 < (int)W) {
-        const Idx o1 = ((Idx)y * W + (Idx)x1) * 3;
-        dst[o1] = __fdiv_rn(acc1[0], acc1[3]);
-        dst[o1 + 1] = __fdiv_rn(acc1[1], acc1[3]);
-        dst[o1 + 2] = __fdiv_rn(acc1[2], acc1[3]);
+    float bright = 0.0f;   // the thread's largest luminance (a NaN never replaces it)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int x = x0 + k * s;
+        if (y0 >= (int)H || x >= (int)W) continue;
+        const float* v = acc[k];
+        const float red = __fdiv_rn(v[0], v[3]), green = __fdiv_rn(v[1], v[3]), blue = __fdiv_rn(v[2], v[3]);
+        dst[(size_t)y0 * W + (size_t)x] = make_float4(-ctr[k][8], red, green, blue);
+        const float l = luminance(red, green, blue);
+        bright = (bright < l) ? l : bright;
+    }
+    if (cells) {
+        // a cell's four columns are two lanes', its four rows four threads'
+        const float o = __shfl_xor_sync(0xffffffffu, bright, 1);
+        bright = (bright < o) ? o : bright;
+        if (h % 2 == 0 && bright > 0.0f)
+            atomicMax(cells + (size_t)(y0 >> (shift + 2)) * cell_pitch + (size_t)(x0 >> (shift + 2)),
+                      __float_as_uint(bright));
     }
 }
 
-// Spacings up to this use the tiled blend; wider ones gather their staged lattice
-// points from scattered sectors and run faster as the direct kernel.
-constexpr int kTiledMaxSpacing = 4;
+// The last level's colours as the caller's image.  Written by the blend itself, twelve bytes a pixel and those sixteen
+// pixels apart, they cost 25 us more than records; this pass over consecutive pixels costs 15-20.
+__global__ void __launch_bounds__(256) atrous_unpack_kernel(const float4* __restrict__ c, size_t npx, float* __restrict__ out)
+{
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i >= npx) return;
+    const float4 v = __ldg(c + i);
+    out[3 * i] = v.y; out[3 * i + 1] = v.z; out[3 * i + 2] = v.w;
+}
 
+// Scratch of a call, in floats: the packed records (eight of normal, position and albedo a pixel, then two arrays of
+// colours that the levels take in turn), then atrous_stats_floats of statistics.
 cudaError_t launch_atrous(const float* pixels, const float* normals, const float* positions, const float* diffuse,
-                          uint32_t W, uint32_t H, float* scratch_a, float* scratch_b, float* tile_stats, float* out,
-                          cudaStream_t st)
+                          uint32_t W, uint32_t H, float* records, float* stats, float* out, cudaStream_t st)
 {
     if (W == 0 || H == 0) return cudaSuccess;
-    const uint32_t tiles = ((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile);
-    // scratch (atrous_stats_floats): per tile kStatsSplit white-point partials, then five
-    // (min, max) |position| ranges per tile, then five (min, max) per image row and tile column
-    float* parts = tile_stats;
-    float2* range = reinterpret_cast<float2*>(tile_stats + (size_t)tiles * kStatsSplit);
-    float2* rrow = range + (size_t)5 * tiles;
-    const uint32_t tiles_x = (W + kTile - 1) / kTile;
-    const uint64_t row_tasks = (uint64_t)H * tiles_x;
-    atrous_row_range_kernel<<<(unsigned)((row_tasks + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, st>>>(
-        positions, W, H, rrow);
-    atrous_tile_range_kernel<<<tiles, 32 * 5, 0, st>>>(rrow, W, H, range);
-    const float* src = pixels;
+    const uint32_t tiles_x = (W + kTile - 1) / kTile, tiles = tiles_x * ((H + kTile - 1) / kTile);
+    const size_t npx = (size_t)W * H;
+    float4* rab = reinterpret_cast<float4*>(records);
+    float4* rc[2] = {rab + 2 * npx, rab + 3 * npx};
+    // per level and tile the white point and the scale of the position term; per level, image row and tile column a
+    // (min, max) |position|; the cells of levels 1-4
+    float* white = stats;
+    float* pos_scale = white + (size_t)5 * tiles;
+    float2* rrow = reinterpret_cast<float2*>(pos_scale + (size_t)5 * tiles);
+    uint32_t* cells = reinterpret_cast<uint32_t*>(rrow + (size_t)5 * H * tiles_x);
+    const size_t nwhite = (size_t)5 * tiles, ncells = atrous_cells(W, H);
+    const uint64_t row_blocks = ((uint64_t)H * tiles_x + kRowWarps - 1) / kRowWarps;
+    const uint64_t pack_blocks = (std::max({npx, nwhite, ncells}) + kPrepareThreads - 1) / kPrepareThreads;
+    atrous_prepare_kernel<<<(unsigned)(3 * std::max(row_blocks, (pack_blocks + 1) / 2)), kPrepareThreads, 0, st>>>(
+        pixels, normals, positions, diffuse, W, H, rab, rc[0], rrow, reinterpret_cast<uint32_t*>(white), nwhite, cells,
+        ncells);
+    atrous_tile_range_kernel<<<tiles, 32 * 5, 0, st>>>(rrow, W, H, pos_scale);
+    bool filled = false;   // whether the level before filled this one's cells
     for (int level = 0; level < 5; ++level) {
-        // ping-pong: in -> A -> B -> A -> B -> out
-        float* dst = level == 4 ? out : ((level % 2 == 0) ? scratch_a : scratch_b);
         const int s = 1 << level;
-        const float2* lrange = range + (size_t)level * tiles;
-        atrous_stats_kernel<<<tiles * kStatsSplit, kStatsThreads, 0, st>>>(src, W, H, s, parts);
-        const bool small = (uint64_t)W * H * 3 < (1ull << 32);
-        if (s <= kTiledMaxSpacing) {
-            // one CTA per kLatX x kLatY tile of each of the s x s sub-lattices
-            const uint32_t lw = (W + s - 1) / s, lh = (H + s - 1) / s;
-            dim3 grid(((lw + kLatX - 1) / kLatX) * s, ((lh + kLatY - 1) / kLatY) * s);
-            if (small)
-                atrous_blend_tiled_kernel<uint32_t><<<grid, kBlendThreads, 0, st>>>(src, normals, positions, diffuse,
-                                                                                   W, H, s, parts, lrange, dst);
-            else
-                atrous_blend_tiled_kernel<size_t><<<grid, kBlendThreads, 0, st>>>(src, normals, positions, diffuse, W,
-                                                                                 H, s, parts, lrange, dst);
+        const float4* src = rc[level % 2];
+        float* lwhite = white + (size_t)level * tiles;
+        if (filled) {
+            atrous_white_kernel<<<(tiles + 3) / 4, 128, 0, st>>>(cells, W, H, s, lwhite);
         } else {
-            dim3 grid((W + 255) / 256, H);
-            if (small)
-                atrous_blend_kernel<uint32_t><<<grid, 256, 0, st>>>(src, normals, positions, diffuse, W, H, s, parts,
-                                                                    lrange, dst);
-            else
-                atrous_blend_kernel<size_t><<<grid, 256, 0, st>>>(src, normals, positions, diffuse, W, H, s, parts,
-                                                                  lrange, dst);
+            // the packed colours start at a record's second float
+            const float* colour = level == 0 ? pixels : reinterpret_cast<const float*>(src) + 1;
+            atrous_stats_kernel<<<tiles * kStatsSplit, kStatsThreads, 0, st>>>(colour, level == 0 ? 3 : 4, W, H, s,
+                                                                              reinterpret_cast<uint32_t*>(lwhite));
         }
-        src = dst;
+        if (level > 0) cells += atrous_level_cells(W, H, 2 * s);
+        filled = level < 4 && whole_footprints(W, H, 2 * s);
+        // one CTA per kLatX x kLatY tile of each of the s x s sub-lattices
+        const uint64_t cols = (uint64_t)((W + s - 1) / s + kLatX - 1) / kLatX * s;
+        const uint64_t blocks = cols * (((H + s - 1) / s + kLatY - 1) / kLatY * s);
+        atrous_blend_kernel<<<(unsigned)blocks, kBlendThreads, 0, st>>>(
+            rab, src, W, H, level, (uint32_t)cols, lwhite, pos_scale + (size_t)level * tiles, rc[(level + 1) % 2],
+            filled ? cells : nullptr, (W + 4 * (uint32_t)s - 1) / (4 * (uint32_t)s));
     }
+    atrous_unpack_kernel<<<(unsigned)((npx + 255) / 256), 256, 0, st>>>(rc[1], npx, out);
     return cudaGetLastError();
 }
 

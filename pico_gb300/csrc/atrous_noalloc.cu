@@ -17,14 +17,13 @@
 //   * at most kNoAllocMaxPixels = 2,097,152 pixels (1920 x 1080 fits) and
 //     65,535 rows per call; larger images are rejected with
 //     PICO_ERR_INVALID_ARG and a message in the context, before any launch;
-//   * the array takes 48 MiB + 5.5 MiB of device memory on each device;
-//   * the output must not overlap any input (the last level writes it while it
-//     still reads the colour and the G-buffer): rejected with PICO_ERR_INVALID_ARG;
+//   * the array takes 128 MiB + 8.8 MiB of device memory on each device;
+//   * the output must not overlap any input: rejected with PICO_ERR_INVALID_ARG;
 //   * every call on a device shares that one array, so calls whose kernels
 //     overlap on the GPU (different streams, or different host threads) race
 //     and corrupt each other's output: order them on one stream or with events;
-//   * nothing in the scratch has to start at zero: each level writes its tile
-//     statistics and its ping-pong image in full before reading them;
+//   * nothing in the scratch has to start at zero: a call clears or writes what it
+//     reads;
 //   * set-up: the first call on a device (with that device current) looks up
 //     the array's address with cudaGetSymbolAddress and caches it; that first
 //     call should come before any stream capture.
@@ -37,25 +36,28 @@
 namespace {
 
 constexpr size_t kNoAllocMaxPixels = size_t(1) << 21;
-constexpr uint32_t kNoAllocMaxRows = 65535;            // the blend kernel's grid.y
+constexpr uint32_t kNoAllocMaxRows = 65535;            // bounds the row ranges' share of the scratch
 // 64 x 64 statistics tiles: ceil(W / 64) * ceil(H / 64).  An image of at most 2^21
 // pixels in at most 64 rows has one tile row of at most 2^21 / 64 tiles (a single
 // row of 2^21 pixels is the worst case); from 65 rows on it has at most 2^21 / 65
 // columns, so at most 505 tiles per tile row and far fewer than 2^15 in all.
 constexpr size_t kNoAllocMaxTiles = kNoAllocMaxPixels / 64;
 static_assert(kNoAllocMaxTiles == 32768, "32,768 statistics tiles");
-constexpr size_t kNoAllocImageFloats = 3 * kNoAllocMaxPixels;
-// The statistics (pico::atrous_stats_floats): 14 floats per tile, and 10 per image row and
-// tile column, of which an accepted image has at most 2^21 / 64 + 65,535 (H * ceil(W / 64)
-// <= W * H / 64 + H).
-constexpr size_t kNoAllocStatsFloats = 14 * kNoAllocMaxTiles + 10 * (kNoAllocMaxPixels / 64 + kNoAllocMaxRows);
-constexpr size_t kNoAllocFloats = 2 * kNoAllocImageFloats + kNoAllocStatsFloats;
+constexpr size_t kNoAllocRecordFloats = 16 * kNoAllocMaxPixels;   // pico::atrous_record_floats
+// The statistics (pico::atrous_stats_floats): 10 floats per tile; 10 per image row and tile
+// column, of which an accepted image has at most 2^21 / 64 + 65,535 (H * ceil(W / 64)
+// <= W * H / 64 + H); and the cells of c x c pixels, c = 4 .. 32, of which it has at most
+// 2^21 / c + 1 each: an image no wider or no higher than c has one row or column of them,
+// otherwise ceil(W / c) * ceil(H / c) < 4 W H / c^2.
+constexpr size_t kNoAllocStatsFloats = 10 * kNoAllocMaxTiles + 10 * (kNoAllocMaxPixels / 64 + kNoAllocMaxRows) +
+                                       (kNoAllocMaxPixels / 4 + kNoAllocMaxPixels / 8 + kNoAllocMaxPixels / 16 +
+                                        kNoAllocMaxPixels / 32 + 4);
+constexpr size_t kNoAllocFloats = kNoAllocRecordFloats + kNoAllocStatsFloats;
 constexpr int kNoAllocMaxDevices = 64;
 
 }  // namespace
 
-// Ping-pong image A, ping-pong image B, then the per-tile statistics (white-point
-// partials and per-level |position| ranges).
+// The packed records, then the statistics (kernels_render.h).
 static __device__ __align__(256) float pico_atrous_noalloc_scratch[kNoAllocFloats];
 
 namespace {
@@ -110,8 +112,7 @@ extern "C" int pico_gpu_atrous_device_noalloc(pico_gpu_ctx* ctx, const float* d_
     if (e == cudaSuccess) e = scratch_for_device(ctx->device, &scratch);
     if (e == cudaSuccess)
         e = launch_atrous(d_pixels, d_normals, d_positions, d_diffuse, width, height, scratch,
-                          scratch + kNoAllocImageFloats, scratch + 2 * kNoAllocImageFloats, d_out,
-                          static_cast<cudaStream_t>(stream));
+                          scratch + kNoAllocRecordFloats, d_out, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_error(ctx, e, "a-trous without allocation");
     return PICO_OK;
 }

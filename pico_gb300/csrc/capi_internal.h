@@ -53,8 +53,8 @@ inline bool ranges_overlap(const float* a, const float* b, size_t n)
     return n != 0 && x < y + bytes && y < x + bytes;
 }
 
-// Whether an a-trous output of W*H*3 floats overlaps any of its four inputs: the
-// last level writes the output while it still reads the colour and the G-buffer.
+// Whether an a-trous output of W*H*3 floats overlaps any of its four inputs, which both
+// device entry points refuse.
 inline bool atrous_output_aliases(const float* out, const float* pixels, const float* normals,
                                   const float* positions, const float* diffuse, size_t n3)
 {

@@ -179,18 +179,24 @@ cudaError_t launch_accumulate(PathBatch& b, uint32_t spb, uint32_t max_samples, 
 cudaError_t launch_stamp(unsigned long long* dst, cudaStream_t st);
 cudaError_t launch_gbuffer(const SceneView& sc, const CameraView& cam, uint32_t W, uint32_t H, float* normals,
                            float* positions, float* diffuse, DeviceStatus* status, int order, cudaStream_t st);
-// Floats of a-trous statistics scratch for a W x H image (beyond its two ping-pong
-// images): per 64 x 64 tile four partial white points (one per CTA of a level's
-// statistics launch) and the five levels' (min, max) |position| ranges, then per
-// image row and tile column the five levels' (min, max) row ranges.
+// Floats of a-trous scratch for a W x H image: the packed records (16 a pixel), and the statistics: per level and
+// 64 x 64 tile a white point and the scale of the position term, per level, image row and tile column the (min, max)
+// |position|, and the luminance cells, c x c pixels each, of levels 1-4 (c = 4, 8, 16, 32).
+inline size_t atrous_record_floats(uint32_t W, uint32_t H) { return (size_t)16 * W * H; }
+inline size_t atrous_level_cells(uint32_t W, uint32_t H, int c) { return (((size_t)W + c - 1) / c) * (((size_t)H + c - 1) / c); }
+inline size_t atrous_cells(uint32_t W, uint32_t H)
+{
+    size_t n = 0;
+    for (int c = 4; c <= 32; c *= 2) n += atrous_level_cells(W, H, c);
+    return n;
+}
 inline size_t atrous_stats_floats(uint32_t W, uint32_t H)
 {
-    const size_t tx = (W + 63) / 64, ty = (H + 63) / 64;
-    return tx * ty * (4 + 5 * 2) + (size_t)5 * 2 * H * tx;
+    const size_t tx = ((size_t)W + 63) / 64, ty = ((size_t)H + 63) / 64;
+    return tx * ty * (5 + 5) + (size_t)5 * 2 * H * tx + atrous_cells(W, H);
 }
 cudaError_t launch_atrous(const float* pixels, const float* normals, const float* positions, const float* diffuse,
-                          uint32_t W, uint32_t H, float* scratch_a, float* scratch_b, float* tile_stats, float* out,
-                          cudaStream_t st);
+                          uint32_t W, uint32_t H, float* records, float* stats, float* out, cudaStream_t st);
 cudaError_t launch_reinhard(float* pixels, uint32_t W, uint32_t H, unsigned* scratch, cudaStream_t st);
 
 }  // namespace pico

@@ -130,12 +130,10 @@ namespace {
 int run_atrous(pico_gpu_ctx* ctx, RenderBuffers& r, const float* d_pix, const float* d_n, const float* d_p,
                const float* d_d, uint32_t W, uint32_t H, float* d_out, cudaStream_t st)
 {
-    const size_t n = (size_t)W * H * 3;
-    cudaError_t e = r.ga.reserve(n * sizeof(float));
-    if (e == cudaSuccess) e = r.gb.reserve(n * sizeof(float));
+    cudaError_t e = r.ga.reserve(atrous_record_floats(W, H) * sizeof(float));
     if (e == cudaSuccess) e = r.stats.reserve(atrous_stats_floats(W, H) * sizeof(float));
     if (e == cudaSuccess)
-        e = launch_atrous(d_pix, d_n, d_p, d_d, W, H, as<float>(r.ga), as<float>(r.gb), as<float>(r.stats), d_out, st);
+        e = launch_atrous(d_pix, d_n, d_p, d_d, W, H, as<float>(r.ga), as<float>(r.stats), d_out, st);
     if (e != cudaSuccess) return cuda_error(ctx, e, "a-trous");
     return PICO_OK;
 }

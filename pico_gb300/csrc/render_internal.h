@@ -13,7 +13,7 @@ struct RenderBuffers {
         senergy, q0, q1, sq, counters;
     pico::DeviceBuffer pixels, variance, count, taken, done, pix_list;
     pico::DeviceBuffer pix_list2, plan;   // exit-aware rounds: the compacted pixel list, the round plan
-    pico::DeviceBuffer gn, gp, gd, ga, gb, stats, out, tonemap;
+    pico::DeviceBuffer gn, gp, gd, ga, stats, out, tonemap;
     pico::DeviceBuffer hdr_pix, hdr_codes, hdr_lens, hdr_off, hdr_body;   // .hdr output: image, codes, their lengths
                                                                           // and places, the file's body
     // radiance cache: training records' queries, throughput and payload, targets; terminal
@@ -31,7 +31,7 @@ struct RenderBuffers {
         for (pico::DeviceBuffer* b : {&org, &dir, &thr, &pay, &hit, &hit_tri, &rng, &depth, &ior_n, &ior_lo, &ior_hi,
                                       &sorg, &sdir, &scontrib, &senergy, &q0, &q1, &sq, &counters, &pixels,
                                       &variance, &count, &taken, &done, &pix_list, &pix_list2, &plan, &gn, &gp, &gd,
-                                      &ga, &gb, &stats,
+                                      &ga, &stats,
                                       &out, &tonemap, &hdr_pix, &hdr_codes, &hdr_lens, &hdr_off, &hdr_body, &nrc_q, &nrc_tp, &nrc_tgt, &nrc_term, &nrc_prev, &nrc_count})
             b->release();
     }
