@@ -621,7 +621,7 @@ def bench_atrous(ctx, args, torch, local):
     algo = ATROUS_BYTES_PER_PIXEL_LEVEL * 5 * W * H
     peak, src = measured_peaks()
     return {"workload": "a-trous, 5 levels, 1920x1080, device buffers, L2 flushed before each call",
-            "ms_per_call": ms, "Mpixels_per_s": W * H / (ms / 1e3) / 1e6, "gpu_launches_per_call": 10,
+            "ms_per_call": ms, "Mpixels_per_s": W * H / (ms / 1e3) / 1e6, "gpu_launches_per_call": 13,
             "roofline": {"bound": "hbm", "achieved": algo / (ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": algo / (ms / 1e3) / 1e9 / peak, "peak_source": src,
                          "algorithmic_bytes_per_call": algo,
@@ -877,7 +877,7 @@ def bench_render_headline(ctx, args, torch, local, dist, world, l2_gbs):
     # kernels per render: extend and shade per depth; per round plan, raygen, accumulate and the
     # compaction (none after the last round); plan set-up, image preparation, G-buffer, a-trous
     rounds = launches // (depth + 1) if launches else 0
-    kernels_per_render = 2 * launches + 4 * rounds - 1 + 2 + 1 + 12
+    kernels_per_render = 2 * launches + 4 * rounds - 1 + 2 + 1 + 13
     out = {"value": value, "ms_per_step": ms, "Mrays_per_s": replica_throughput(rays, world, ms / 1e3),
            "samples_per_render": st["samples"], "rays_per_render": {k: st[k] for k in (
                "camera_paths", "bounce_rays", "shadow_rays", "gbuffer_rays")},
