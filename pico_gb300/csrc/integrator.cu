@@ -1194,12 +1194,12 @@ cudaError_t launch_prepare_image(const uint32_t* count, uint32_t W, uint32_t H, 
 cudaError_t launch_gbuffer(const SceneView& sc, const CameraView& cam, uint32_t W, uint32_t H, float* normals,
                            float* positions, float* diffuse, DeviceStatus* status, int order, cudaStream_t st)
 {
-    const cudaError_t e = cudaMemsetAsync(&status->work, 0, sizeof(unsigned long long), st);
+    const cudaError_t e = cudaMemsetAsync(&status->gbuffer_work, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     with_variant(order, sc, [&](auto v) {
         constexpr int V = decltype(v)::value;
         gbuffer_kernel<V><<<grid_for(gbuffer_kernel<V>, W * H, 128), 128, 0, st>>>(
-            sc, cam, W, H, normals, positions, diffuse, &status->work, &status->trace_error);
+            sc, cam, W, H, normals, positions, diffuse, &status->gbuffer_work, &status->trace_error);
     });
     return cudaGetLastError();
 }

@@ -13,7 +13,8 @@ namespace pico {
 struct DeviceStatus {
     int trace_error;                 // TraceStatus bits
     int pad[3];
-    unsigned long long work;         // persistent-kernel work counter
+    unsigned long long work;         // claims of a ray batch's launch (launch_trace)
+    unsigned long long gbuffer_work; // claims of the G-buffer's launch, which may run beside a ray batch on another stream
     unsigned long long counters[4];  // nodes, triangles, instances, spare
     unsigned long long rays[4];      // render tallies: camera, bounce, shadow rays traced; spare
 };
