@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kBlendThreads, 6) atrous_blend_kernel(
                 const float da = fmaf(az, az, vv.x) + vv.y;
                 const float e = fmaf(da, iw[k], fmaf(np.y, ip[k], fmaf(np.x, -4.0f * kLog2e, kAtrousLog2[j * 5 + i])));
                 float w;
-                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(e));
+                asm("ex2.approx.f32 %0, %1;" : "=f"(w) : "f"(e));   // keeps subnormal weights
                 acc[k][0] = fmaf(c.y, w, acc[k][0]);
                 acc[k][1] = fmaf(c.z, w, acc[k][1]);
                 acc[k][2] = fmaf(c.w, w, acc[k][2]);
