@@ -319,6 +319,9 @@ static bool whole_footprints(uint32_t W, uint32_t H, int s)
 // At spacing s every tap of a pixel lands on the pixel's own sub-lattice (x mod s, y mod s), so a CTA takes a
 // kLatX x kLatY tile of one sub-lattice at every spacing; the (kLatX + 4) x (kLatY + 4) lattice points its taps read
 // (coordinates clamped exactly as the taps clamp them) are copied to shared memory once, asynchronously and past L1.
+// Points that only pixels outside the image would read are left out: of a small image at a large spacing they were
+// most of a footprint, all clamped to the same few border pixels (65 x 40, spacing 16: 33 us with them, 6 without;
+// 1601 x 901 whole: 433 us and 387).
 // Each thread blends two neighbouring columns, whose taps overlap, and reads each record once for both; the records of
 // a footprint row are split into even and odd columns so that a warp's loads hit consecutive records.
 //
@@ -352,13 +355,14 @@ __global__ void __launch_bounds__(kBlendThreads, 6) atrous_blend_kernel(
     const int lx0 = tx * kLatX - 2, ly0 = ty * kLatY - 2;   // lattice coordinate of footprint entry (0, 0)
     int ex = (int)threadIdx.x % kFootX, ey = (int)threadIdx.x / kFootX;
     for (int e = (int)threadIdx.x; e < kFootX * kFootY; e += kBlendThreads) {
-        const int x = clampi(rx + (lx0 + ex) * s, 0, (int)W - 1);
-        const int y = clampi(ry + (ly0 + ey) * s, 0, (int)H - 1);
-        const size_t f = (size_t)y * W + (size_t)x;
-        float4* slot = rec + 3 * ((ey * 2 + (ex & 1)) * kHalfX + (ex >> 1));
-        copy16(slot, rab + 2 * f);
-        copy16(slot + 1, rab + 2 * f + 1);
-        copy16(slot + 2, rc + f);
+        const int x = rx + (lx0 + ex) * s, y = ry + (ly0 + ey) * s;
+        if (x < (int)W + 2 * s && y < (int)H + 2 * s) {   // beyond that, only points outside the image read it
+            const size_t f = (size_t)clampi(y, 0, (int)H - 1) * W + (size_t)clampi(x, 0, (int)W - 1);
+            float4* slot = rec + 3 * ((ey * 2 + (ex & 1)) * kHalfX + (ex >> 1));
+            copy16(slot, rab + 2 * f);
+            copy16(slot + 1, rab + 2 * f + 1);
+            copy16(slot + 2, rc + f);
+        }
         ex += kBlendThreads % kFootX;
         ey += kBlendThreads / kFootX;
         if (ex >= kFootX) { ex -= kFootX; ++ey; }
