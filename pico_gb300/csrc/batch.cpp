@@ -71,6 +71,7 @@ struct Params {
 struct Prepared {
     uint32_t W = 0, H = 0;
     size_t npx = 0, nactive = 0;
+    bool fresh = false;   // CountScan
     CameraView cam{};
 };
 
@@ -170,6 +171,7 @@ cudaError_t upload_render(const pico_render_item& it, BatchSlot& s, Prepared& pr
     pr.npx = (size_t)pr.W * pr.H;
     const CountScan scan = scan_counts(it.sample_count, pr.npx, cfg.max_samples);
     pr.nactive = scan.unfinished;
+    pr.fresh = scan.fresh;
     pr.cam = make_camera_view(it.camera);
     cudaError_t e = r.pixels.reserve(pr.npx * 3 * sizeof(float));
     if (e == cudaSuccess) e = r.variance.reserve(pr.npx * 3 * sizeof(float));
@@ -407,6 +409,7 @@ int run_batch(pico_gpu_ctx* ctx, uint32_t n, const pico_render_item* items, cons
     const auto t_run = clock::now();
     e = cudaGraphLaunch(exec, st);
     for (uint32_t r = 0; r < n && e == cudaSuccess; ++r) {   // while the graph runs
+        if (!prep[r].fresh) continue;   // the pages of a render that goes on were there to be read
         populate_for_writing(items[r].pixels_rgb, prep[r].npx * 3 * sizeof(float));
         populate_for_writing(items[r].variance_rgb, prep[r].npx * 3 * sizeof(float));
         populate_for_writing(items[r].sample_count, prep[r].npx * sizeof(uint32_t));

@@ -95,15 +95,22 @@ cudaError_t reserve_paths(RenderBuffers& r, size_t n)
     return e;
 }
 
+bool no_samples(const uint32_t* count, size_t npx)
+{
+    constexpr size_t kBlock = 1024;   // the loop inside is vectorised
+    for (size_t p0 = 0; p0 < npx; p0 += kBlock) {
+        uint32_t any = 0;
+        for (size_t p = p0; p < std::min(npx, p0 + kBlock); ++p) any |= count[p];
+        if (any) return false;
+    }
+    return npx > 0;
+}
+
 CountScan scan_counts(const uint32_t* count, size_t npx, uint32_t max_samples)
 {
     size_t unfinished = 0;
-    uint32_t any = 0;
-    for (size_t p = 0; p < npx; ++p) {
-        unfinished += count[p] < max_samples ? 1u : 0u;
-        any |= count[p];
-    }
-    return CountScan{unfinished, npx > 0 && any == 0 && max_samples > 0};
+    for (size_t p = 0; p < npx; ++p) unfinished += count[p] < max_samples ? 1u : 0u;
+    return CountScan{unfinished, max_samples > 0 && unfinished == npx && no_samples(count, npx)};
 }
 
 PathBatch make_batch(RenderBuffers& r, uint32_t n, uint32_t npix, uint32_t W, const uint32_t* pix_list)
@@ -493,8 +500,11 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
     // finished ones there.  The radiance cache's passes take a compacted list, which is built here when some pixels
     // are finished.  A fresh render's mean and variance are not uploaded (accumulate replaces them with a pixel's
     // first sample): the caller's pages, often untouched, are then faulted in once, by the download, instead of twice.
-    const CountScan scan = scan_counts(sample_count, npx, cfg->max_samples);
+    // Only the cache's renders count the pixels left; for the others the host reads no further than the first sample.
     const bool with_cache = cfg->estimator == PICO_ESTIMATOR_RADIANCE_CACHE;
+    CountScan scan;
+    if (with_cache) scan = scan_counts(sample_count, npx, cfg->max_samples);
+    else scan.fresh = cfg->max_samples > 0 && no_samples(sample_count, npx);
     const bool host_list = with_cache && scan.unfinished < npx;
     std::vector<uint32_t> active, done;
     if (host_list) {
@@ -531,9 +541,10 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
     bool cancelled = false;
     const size_t nactive = with_cache ? scan.unfinished : npx;
     if (nactive > 0 && cfg->max_samples > 0) {
-        r.results = {{pixels, npx * 3 * sizeof(float)},
-                     {variance, npx * 3 * sizeof(float)},
-                     {sample_count, npx * sizeof(uint32_t)}};
+        if (scan.fresh)   // the pages of a render that goes on were there to be read
+            r.results = {{pixels, npx * 3 * sizeof(float)},
+                         {variance, npx * 3 * sizeof(float)},
+                         {sample_count, npx * sizeof(uint32_t)}};
         status = with_cache
                      ? render_with_cache(ctx, scene, ctx->cache, cfg, cam, r, nactive, should_quit, cancelled)
                      : run_sample_batches(ctx, scene, cfg, cam, r, nactive, as<float>(r.pixels),

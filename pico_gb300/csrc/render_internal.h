@@ -55,6 +55,8 @@ struct CountScan {
     size_t unfinished = 0;   // pixels that will take samples
     bool fresh = false;      // no pixel has a sample and all will take one: the mean and variance passed in are not read
 };
+// Whether no pixel has a sample (false for no pixels): reads up to the first sample.
+bool no_samples(const uint32_t* count, size_t npx);
 CountScan scan_counts(const uint32_t* count, size_t npx, uint32_t max_samples);
 
 template <class T>
