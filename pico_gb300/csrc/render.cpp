@@ -418,25 +418,27 @@ int run_sample_batches(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pic
 }
 
 // A cancelled render whose mean and variance were not uploaded: the device buffers get the caller's values for the
-// pixels without a sample.
+// pixels without a sample, run by run (the path limit's chunks leave bands of them), with no host memory taken.
 cudaError_t restore_unsampled(RenderBuffers& r, const float* pixels, const float* variance, size_t npx, cudaStream_t st)
 {
-    std::vector<uint32_t> count(npx);
-    std::vector<float> mean(3 * npx), var(3 * npx);
-    cudaError_t e = cudaMemcpyAsync(count.data(), r.count.ptr, npx * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(mean.data(), r.pixels.ptr, 3 * npx * sizeof(float), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(var.data(), r.variance.ptr, 3 * npx * sizeof(float), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return e;
-    for (size_t p = 0; p < npx; ++p)
-        if (count[p] == 0)
-            for (size_t k = 3 * p; k < 3 * p + 3; ++k) {
-                mean[k] = pixels[k];
-                var[k] = variance[k];
-            }
-    e = cudaMemcpyAsync(r.pixels.ptr, mean.data(), 3 * npx * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r.variance.ptr, var.data(), 3 * npx * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the host vectors end with this call
+    constexpr size_t kBlock = 4096;
+    uint32_t count[kBlock];
+    float *mean = as<float>(r.pixels), *var = as<float>(r.variance);
+    cudaError_t e = cudaSuccess;
+    for (size_t p0 = 0; p0 < npx && e == cudaSuccess; p0 += kBlock) {
+        const size_t n = std::min(kBlock, npx - p0);
+        e = cudaMemcpyAsync(count, as<uint32_t>(r.count) + p0, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        for (size_t k = 0; k < n && e == cudaSuccess;) {
+            if (count[k] != 0) { ++k; continue; }
+            size_t end = k + 1;
+            while (end < n && count[end] == 0) ++end;
+            const size_t at = 3 * (p0 + k), bytes = 3 * (end - k) * sizeof(float);
+            e = cudaMemcpyAsync(mean + at, pixels + at, bytes, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(var + at, variance + at, bytes, cudaMemcpyHostToDevice, st);
+            k = end;
+        }
+    }
     return e;
 }
 
@@ -541,15 +543,16 @@ int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_c
     bool cancelled = false;
     const size_t nactive = with_cache ? scan.unfinished : npx;
     if (nactive > 0 && cfg->max_samples > 0) {
-        if (scan.fresh)   // the pages of a render that goes on were there to be read
-            r.results = {{pixels, npx * 3 * sizeof(float)},
-                         {variance, npx * 3 * sizeof(float)},
-                         {sample_count, npx * sizeof(uint32_t)}};
+        if (scan.fresh) {   // the pages of a render that goes on were there to be read
+            r.results[0] = {pixels, npx * 3 * sizeof(float)};
+            r.results[1] = {variance, npx * 3 * sizeof(float)};
+            r.results[2] = {sample_count, npx * sizeof(uint32_t)};
+        }
         status = with_cache
                      ? render_with_cache(ctx, scene, ctx->cache, cfg, cam, r, nactive, should_quit, cancelled)
                      : run_sample_batches(ctx, scene, cfg, cam, r, nactive, as<float>(r.pixels),
                                           as<float>(r.variance), as<uint32_t>(r.count), should_quit, st, cancelled);
-        r.results.clear();
+        r.forget_results();
         if (status != PICO_OK) return status;
     }
     status = take_device_status(ctx, st);

@@ -4,9 +4,6 @@
 #include "capi_internal.h"
 #include "kernels_render.h"
 
-#include <utility>
-#include <vector>
-
 // Path state and image buffers of one render, grown on demand.
 struct RenderBuffers {
     pico::DeviceBuffer org, dir, thr, pay, hit, hit_tri, rng, depth, ior_n, ior_lo, ior_hi, sorg, sdir, scontrib,
@@ -20,11 +17,15 @@ struct RenderBuffers {
     // queries; previous roughness per path; entry counters
     pico::DeviceBuffer nrc_q, nrc_tp, nrc_tgt, nrc_term, nrc_prev, nrc_count;
     // the host buffers this render's results will go to, populated once the device has its first work
-    std::vector<std::pair<void*, size_t>> results;
+    struct { void* p; size_t bytes; } results[3] = {};
+    void forget_results()
+    {
+        for (auto& b : results) b = {};
+    }
     void populate_results()
     {
-        for (const auto& b : results) pico::populate_for_writing(b.first, b.second);
-        results.clear();
+        for (const auto& b : results) pico::populate_for_writing(b.p, b.bytes);
+        forget_results();
     }
     ~RenderBuffers()
     {
