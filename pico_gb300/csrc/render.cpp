@@ -67,6 +67,9 @@ CameraView make_camera_view(const pico_camera& c)
     return v;
 }
 
+// For tests: the most bytes that the buffers of a radiance-cache render may grow to.
+extern "C" void pico_test_cache_budget(pico_gpu_ctx* ctx, uint64_t bytes) { render_buffers(ctx)->budget = (size_t)bytes; }
+
 RenderBuffers* render_buffers(pico_gpu_ctx* ctx)
 {
     if (!ctx->render) ctx->render = new RenderBuffers();
@@ -82,16 +85,24 @@ void free_render_buffers(pico_gpu_ctx* ctx)
     ctx->shade_timer = nullptr;
 }
 
+// f(buffer, bytes) for every buffer of the state of n paths.
+template <class F>
+static void for_path_buffers(RenderBuffers& r, size_t n, F&& f)
+{
+    for (DeviceBuffer* b : {&r.org, &r.dir, &r.thr, &r.pay, &r.hit, &r.sorg, &r.sdir, &r.scontrib, &r.senergy,
+                            &r.ior_lo, &r.ior_hi})
+        f(*b, n * sizeof(float4));
+    for (DeviceBuffer* b : {&r.hit_tri, &r.depth, &r.ior_n, &r.q0, &r.q1, &r.sq}) f(*b, n * sizeof(uint32_t));
+    f(r.rng, n * sizeof(unsigned long long));
+    f(r.counters, kDepthRing * sizeof(DepthQueues));
+}
+
 cudaError_t reserve_paths(RenderBuffers& r, size_t n)
 {
     cudaError_t e = cudaSuccess;
-    for (DeviceBuffer* b : {&r.org, &r.dir, &r.thr, &r.pay, &r.hit, &r.sorg, &r.sdir, &r.scontrib, &r.senergy,
-                            &r.ior_lo, &r.ior_hi})
-        if (e == cudaSuccess) e = b->reserve(n * sizeof(float4));
-    for (DeviceBuffer* b : {&r.hit_tri, &r.depth, &r.ior_n, &r.q0, &r.q1, &r.sq})
-        if (e == cudaSuccess) e = b->reserve(n * sizeof(uint32_t));
-    if (e == cudaSuccess) e = r.rng.reserve(n * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = r.counters.reserve(kDepthRing * sizeof(DepthQueues));
+    for_path_buffers(r, n, [&](DeviceBuffer& b, size_t bytes) {
+        if (e == cudaSuccess) e = b.reserve(bytes);
+    });
     return e;
 }
 
@@ -156,6 +167,48 @@ static uint32_t path_limit(const pico_gpu_ctx* ctx) { return ctx->max_paths ? ct
 // most as many passes together, with or without a flag.
 constexpr uint32_t kCancelSamplesPerBatch = 16;
 
+// f(buffer, bytes) for every buffer of a group of passes.  The records' queries and the camera paths' share one buffer
+// in a group of one pass: its optimiser steps are enqueued before its camera paths.
+template <class F>
+void for_cache_buffers(RenderBuffers& r, uint32_t group, uint32_t chunk_pix, uint32_t ntrain, uint32_t rec_cap, F&& f)
+{
+    const size_t slots = (size_t)group * std::max<size_t>(chunk_pix, ntrain);
+    const size_t records = (size_t)group * rec_cap, terms = (size_t)group * chunk_pix;
+    for_path_buffers(r, slots, f);
+    f(r.nrc_q, (group == 1 ? std::max(records, terms) : records) * sizeof(pico_nrc_query));
+    f(r.nrc_tp, records * 2 * sizeof(float4));
+    f(r.nrc_tgt, records * sizeof(float4));
+    if (group > 1) f(r.nrc_term, terms * sizeof(pico_nrc_query));
+    f(r.nrc_prev, slots * sizeof(float));
+    f(r.nrc_count, 2 * kCancelSamplesPerBatch * sizeof(uint32_t));
+}
+
+// Reserves a group's buffers, halving the group (down to one pass) where they would take more than half of the
+// device's free memory (the denoiser's buffers come after them, and a context keeps its own) or do not fit.  What a
+// group that did not fit had reserved is given back before the next is tried.
+cudaError_t reserve_cache_group(RenderBuffers& r, uint32_t& group, uint32_t chunk_pix, uint32_t ntrain,
+                                uint32_t rec_cap)
+{
+    for (bool last = false;; last = group == 1, group = std::max(1u, group / 2)) {
+        size_t more = 0, held = 0, free_bytes = 0, total = 0;
+        for_cache_buffers(r, group, chunk_pix, ntrain, rec_cap, [&](DeviceBuffer& b, size_t bytes) {
+            more += bytes > b.cap ? bytes - b.cap : 0;
+            held += b.cap;
+        });
+        if (group > 1 && more > 0 && cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && more > free_bytes / 2) continue;
+        cudaError_t e = cudaSuccess;
+        for_cache_buffers(r, group, chunk_pix, ntrain, rec_cap, [&](DeviceBuffer& b, size_t bytes) {
+            if (e != cudaSuccess || bytes <= b.cap) return;
+            const size_t before = b.cap;
+            e = held - before + bytes > r.budget ? cudaErrorMemoryAllocation : b.reserve(bytes);
+            held += b.cap - before;
+        });
+        if (e != cudaErrorMemoryAllocation || last) return e;
+        cudaGetLastError();
+        for_cache_buffers(r, 2, 0, 0, 0, [](DeviceBuffer& b, size_t) { b.release(); });
+    }
+}
+
 // PICO_ESTIMATOR_RADIANCE_CACHE: warmup_frames training-only passes, then per
 // sample pass the cache trains on train_paths full-depth physical paths (at most
 // max_train_steps optimiser steps of at most train_batch records, spread over all
@@ -184,19 +237,7 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
     const uint32_t room = std::min(path_limit(ctx), 1u << 24);
     uint32_t group = std::max(1u, std::min({kCancelSamplesPerBatch, passes, (1u << 24) / std::max(rec_cap, 1u),
                                             chunk_pix < nactive ? 1u : room / std::max({chunk_pix, ntrain, 1u})}));
-    cudaError_t e = cudaSuccess;
-    for (;; group /= 2) {
-        const size_t slots = (size_t)group * std::max<size_t>(chunk_pix, ntrain);
-        e = reserve_paths(r, slots);
-        if (e == cudaSuccess) e = r.nrc_q.reserve((size_t)group * rec_cap * sizeof(pico_nrc_query));
-        if (e == cudaSuccess) e = r.nrc_tp.reserve((size_t)group * rec_cap * 2 * sizeof(float4));
-        if (e == cudaSuccess) e = r.nrc_tgt.reserve((size_t)group * rec_cap * sizeof(float4));
-        if (e == cudaSuccess) e = r.nrc_term.reserve((size_t)group * chunk_pix * sizeof(pico_nrc_query));
-        if (e == cudaSuccess) e = r.nrc_prev.reserve(slots * sizeof(float));
-        if (e == cudaSuccess) e = r.nrc_count.reserve(2 * kCancelSamplesPerBatch * sizeof(uint32_t));
-        if (e != cudaErrorMemoryAllocation || group == 1) break;
-        cudaGetLastError();
-    }
+    cudaError_t e = reserve_cache_group(r, group, chunk_pix, ntrain, rec_cap);
     if (e != cudaSuccess) return cuda_error(ctx, e, "radiance cache render buffers");
     if (!(c->hi[0] > c->lo[0] || c->hi[1] > c->lo[1] || c->hi[2] > c->lo[2]))
         nrc::set_geometry(c, scene->view.tlas_fast_lo, scene->view.tlas_fast_hi);
@@ -210,7 +251,7 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
     rec.count = as<uint32_t>(r.nrc_count);
     term.mode = kNrcTerminate;
     term.capacity = chunk_pix;
-    term.queries = as<float4>(r.nrc_term);
+    term.queries = as<float4>(group > 1 ? r.nrc_term : r.nrc_q);
     term.count = as<uint32_t>(r.nrc_count) + kCancelSamplesPerBatch;
     term.prev_rough = as<float>(r.nrc_prev);
     term.geo = c->geo;
@@ -262,7 +303,8 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
         const bool sampling = pass >= c->cfg.warmup_frames;
         const uint32_t n = std::min(group, (sampling ? passes : c->cfg.warmup_frames) - pass);
         if (training) {
-            const int status = trace_training(n);
+            int status = trace_training(n);
+            if (status == PICO_OK) status = train_pass(0);   // before the camera paths: for_cache_buffers
             if (status != PICO_OK) return status;
         }
         // one sample per active pixel and pass, ending in the cache
@@ -276,7 +318,7 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
                                        order, st);
             }
             for (uint32_t k = 0; k < n && e == cudaSuccess; ++k) {
-                if (training && p0 == 0) {
+                if (training && p0 == 0 && k > 0) {
                     const int status = train_pass(k);
                     if (status != PICO_OK) return status;
                 }

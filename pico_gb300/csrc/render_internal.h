@@ -16,6 +16,7 @@ struct RenderBuffers {
     // radiance cache: training records' queries, throughput and payload, targets; terminal
     // queries; previous roughness per path; entry counters
     pico::DeviceBuffer nrc_q, nrc_tp, nrc_tgt, nrc_term, nrc_prev, nrc_count;
+    size_t budget = ~size_t(0);   // pico_test_cache_budget
     // the host buffers this render's results will go to, populated once the device has its first work
     struct { void* p; size_t bytes; } results[3] = {};
     void forget_results()
