@@ -120,8 +120,12 @@ bool no_samples(const uint32_t* count, size_t npx)
 CountScan scan_counts(const uint32_t* count, size_t npx, uint32_t max_samples)
 {
     size_t unfinished = 0;
-    for (size_t p = 0; p < npx; ++p) unfinished += count[p] < max_samples ? 1u : 0u;
-    return CountScan{unfinished, max_samples > 0 && unfinished == npx && no_samples(count, npx)};
+    uint32_t any = 0;
+    for (size_t p = 0; p < npx; ++p) {
+        unfinished += count[p] < max_samples ? 1u : 0u;
+        any |= count[p];
+    }
+    return CountScan{unfinished, npx > 0 && any == 0 && max_samples > 0};
 }
 
 PathBatch make_batch(RenderBuffers& r, uint32_t n, uint32_t npix, uint32_t W, const uint32_t* pix_list)
