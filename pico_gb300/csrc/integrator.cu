@@ -663,7 +663,19 @@ __global__ void __launch_bounds__(kRenderThreads, kShadeBlocksPerSm) shade_physi
         block_append(r, cont, &next->paths, shadow, &next->shadows, app, at, sat);
         if (cont) b.queue[nxt][at] = i;
         if (shadow) b.shadow_queue[sat] = i;
-        if (nrc.mode != kNrcOff) {
+        if (nrc.mode == kNrcRecord && emit) {
+            const uint32_t pass = i / nrc.pass_paths;
+            const uint64_t e = (uint64_t)depth * nrc.pass_paths + (i - pass * nrc.pass_paths);
+            if (e < nrc.capacity) {   // records end before max_depth, so every one has its place
+                const size_t entry = (size_t)pass * nrc.capacity + e;
+                float4* q = nrc.queries + 4 * entry;
+                q[0] = eq[0]; q[1] = eq[1]; q[2] = eq[2]; q[3] = eq[3];
+                nrc.rec_tp[2 * entry] = et;
+                nrc.rec_tp[2 * entry + 1] = ep;
+                nrc.written[pass * record_flags(nrc.capacity) + e] = 1;
+            }
+        }
+        if (nrc.mode == kNrcTerminate) {
             // an entry in its path's pass: one atomic per pass that the warp's paths belong to
             const unsigned emits = __ballot_sync(0xffffffffu, emit);
             if (emit) {
@@ -674,13 +686,8 @@ __global__ void __launch_bounds__(kRenderThreads, kShadeBlocksPerSm) shade_physi
                 if (lane == leader) ea = atomicAdd(nrc.count + pass, (uint32_t)__popc(peers));
                 ea = __shfl_sync(peers, ea, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
                 if (ea < nrc.capacity) {
-                    const size_t entry = (size_t)pass * nrc.capacity + ea;
-                    float4* q = nrc.queries + 4 * entry;
+                    float4* q = nrc.queries + 4 * ((size_t)pass * nrc.capacity + ea);
                     q[0] = eq[0]; q[1] = eq[1]; q[2] = eq[2]; q[3] = eq[3];
-                    if (nrc.mode == kNrcRecord) {
-                        nrc.rec_tp[2 * entry] = et;
-                        nrc.rec_tp[2 * entry + 1] = ep;
-                    }
                 }
             }
         }
@@ -719,21 +726,72 @@ __global__ void __launch_bounds__(kRenderThreads) train_raygen_kernel(PathBatch 
     }
 }
 
+// The order of a pass's records (NrcShadeArgs::order), in two launches of one CTA per pass (y) and kRecordSegment
+// entries (x): how many entries each segment has, then their list from the segments' counts before it on.  Both are
+// short beside their launches (3 and 4 us for four passes of 65,536 paths and depth 8); computing the targets in the
+// second as well took 30 us, the entries being sparse, against 11 in a launch over the list.
+__device__ __forceinline__ uint4 record_written(const NrcShadeArgs& nrc)
+{
+    const size_t at = (size_t)blockIdx.x * kRecordSegment + 16 * threadIdx.x, n = record_flags(nrc.capacity);
+    return at < n ? *reinterpret_cast<const uint4*>(nrc.written + blockIdx.y * n + at) : make_uint4(0u, 0u, 0u, 0u);
+}
+__device__ __forceinline__ uint32_t flag_count(uint4 w) { return __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w); }
+// The sum of v over the block's threads, and of those before this one in `before`.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t& before)
+{
+    __shared__ uint32_t warp_sum[kRenderThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t sum = v;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, sum, d);
+        if ((int)lane >= d) sum += u;
+    }
+    __syncthreads();   // an earlier call's sums have been read
+    if (lane == 31) warp_sum[warp] = sum;
+    __syncthreads();
+    uint32_t total = 0;
+    before = sum - v;
+    for (uint32_t w = 0; w < kRenderThreads / 32; ++w) {
+        if (w < warp) before += warp_sum[w];
+        total += warp_sum[w];
+    }
+    return total;
+}
+__global__ void __launch_bounds__(kRenderThreads) nrc_count_records_kernel(NrcShadeArgs nrc)
+{
+    uint32_t before;
+    const uint32_t total = block_scan(flag_count(record_written(nrc)), before);
+    if (threadIdx.x == 0) nrc.segments[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(kRenderThreads) nrc_order_records_kernel(NrcShadeArgs nrc)
+{
+    const uint32_t* segments = nrc.segments + (size_t)blockIdx.y * gridDim.x;
+    uint32_t earlier = 0, before;
+    for (uint32_t s = threadIdx.x; s < blockIdx.x; s += kRenderThreads) earlier += segments[s];
+    earlier = block_scan(earlier, before);
+    const uint4 w = record_written(nrc);
+    const uint32_t total = block_scan(flag_count(w), before);
+    if (threadIdx.x == 0 && blockIdx.x + 1 == gridDim.x) nrc.count[blockIdx.y] = earlier + total;
+    uint32_t* out = nrc.order + (size_t)blockIdx.y * nrc.capacity + earlier + before;
+    const uint32_t first = blockIdx.x * kRecordSegment + 16 * threadIdx.x, words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (uint32_t k = 0; k < 16; ++k)
+        if ((words[k / 4] >> (8 * (k % 4))) & 1u) *out++ = first + k;
+}
+static_assert(kRecordSegment == 16 * kRenderThreads, "16 entries a thread");
+
 // Target of each training record: (final payload - payload on arrival) / throughput
 // on arrival, per channel (0 where the throughput is 0); NaN for a path whose
 // payload is not finite, which training skips.
-__global__ void __launch_bounds__(kRenderThreads) nrc_targets_kernel(const float4* __restrict__ queries,
-                                                                    const float4* __restrict__ rec_tp,
-                                                                    const float4* __restrict__ pay,
-                                                                    const uint32_t* count, uint32_t passes,
-                                                                    uint32_t capacity, float4* targets)
+__global__ void __launch_bounds__(kRenderThreads) nrc_targets_kernel(NrcShadeArgs nrc, const float4* __restrict__ pay,
+                                                                    float4* targets)
 {
-    for (uint32_t p = 0; p < passes; ++p) {
-        const uint32_t n = min(count[p], capacity);
+    for (uint32_t p = 0; p < nrc.passes; ++p) {
+        const uint32_t n = nrc.count[p];
         for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-            const size_t j = (size_t)p * capacity + k;
-            const uint32_t path = __float_as_uint(queries[4 * j + 3].y);
-            const float4 T = rec_tp[2 * j], P = rec_tp[2 * j + 1], F = pay[path];
+            const size_t j = (size_t)p * nrc.capacity + nrc.order[(size_t)p * nrc.capacity + k];
+            const uint32_t path = __float_as_uint(nrc.queries[4 * j + 3].y);
+            const float4 T = nrc.rec_tp[2 * j], P = nrc.rec_tp[2 * j + 1], F = pay[path];
             float4 t;
             t.x = T.x > 0.0f ? (F.x - P.x) / T.x : 0.0f;
             t.y = T.y > 0.0f ? (F.y - P.y) / T.y : 0.0f;
@@ -1101,14 +1159,17 @@ cudaError_t launch_training_paths(const SceneView& sc, PathBatch& b, const Camer
     PathBatch t = b;
     t.n = nrc.passes * nrc.pass_paths;
     cudaError_t e = cudaMemsetAsync(t.depths, 0, kDepthRing * sizeof(DepthQueues), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(nrc.count, 0, nrc.passes * sizeof(uint32_t), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(nrc.written, 0, nrc.passes * record_flags(nrc.capacity), st);
     if (e != cudaSuccess) return e;
     train_raygen_kernel<<<grid_for(train_raygen_kernel, t.n, kRenderThreads), kRenderThreads, 0, st>>>(
         t, cam, seed, frame, nrc.pass_paths, W, W * H);
     e = run_depth_loop(sc, t, max_depth, true, nrc, status, order, st);
     if (e != cudaSuccess) return e;
+    const dim3 segments((unsigned)record_segments(nrc.capacity), nrc.passes);
+    nrc_count_records_kernel<<<segments, kRenderThreads, 0, st>>>(nrc);
+    nrc_order_records_kernel<<<segments, kRenderThreads, 0, st>>>(nrc);
     nrc_targets_kernel<<<grid_for(nrc_targets_kernel, nrc.capacity, kRenderThreads), kRenderThreads, 0, st>>>(
-        nrc.queries, nrc.rec_tp, t.pay, nrc.count, nrc.passes, nrc.capacity, targets);
+        nrc, t.pay, targets);
     return cudaGetLastError();
 }
 

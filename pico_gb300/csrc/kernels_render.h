@@ -122,6 +122,9 @@ struct RenderProbe {
 //                  vertex's query; the cache's answer times the throughput is
 //                  added to the payload after the depth loop.
 enum NrcMode { kNrcOff = 0, kNrcRecord = 1, kNrcTerminate = 2 };
+constexpr uint32_t kRecordSegment = 4096;   // entries of a CTA of the ordering kernels, 16 a thread
+inline size_t record_segments(uint32_t capacity) { return ((size_t)capacity + kRecordSegment - 1) / kRecordSegment; }
+PICO_HD size_t record_flags(uint32_t capacity) { return ((size_t)capacity + 15) & ~(size_t)15; }
 struct NrcShadeArgs {
     int mode;
     uint32_t passes;          // passes traced together, pass p on paths [p * pass_paths, (p + 1) * pass_paths)
@@ -129,8 +132,14 @@ struct NrcShadeArgs {
     uint32_t capacity;        // entries of queries / rec_tp per pass
     uint32_t bounces;         // kNrcTerminate: bounces before the cache answers (one more behind a glossy vertex)
     float4* queries;          // 4 float4 per entry (pico_nrc_query); pass p's from entry p * capacity on
-    float4* rec_tp;           // kNrcRecord: 2 float4 per entry
-    uint32_t* count;          // entries appended, per pass
+    uint32_t* count;          // entries, per pass
+    // kNrcRecord: 2 float4 per entry.  A record's entry is its depth and path (depth * pass_paths + the path's number
+    // in its pass), whichever thread shades it first, and order lists the entries written, ascending: a training step's
+    // records do not depend on the order in which they arrive.
+    float4* rec_tp;
+    uint8_t* written;         // per entry 0 or 1; pass p's from p * record_flags(capacity) on
+    uint32_t* segments;       // per pass and kRecordSegment entries: how many are written
+    uint32_t* order;          // pass p's from p * capacity on
     float* prev_rough;        // kNrcTerminate: per path, roughness of its previous vertex
     // the cache the terminating paths query
     nrc::GridGeometry geo;
@@ -162,7 +171,7 @@ cudaError_t launch_prepare_image(const uint32_t* count, uint32_t W, uint32_t H, 
 // The radiance cache's training paths of nrc.passes sample passes: nrc.pass_paths
 // full-depth physical paths each, from pseudo-random pixels of the W x H image (path
 // slots of b from 0 on; pass p draws with frame + p), recording every shaded vertex
-// (kNrcRecord), then the records' targets (4 floats each) in `targets`.
+// (kNrcRecord), then the records' order and their targets (4 floats an entry) in `targets`.
 cudaError_t launch_training_paths(const SceneView& sc, PathBatch& b, const CameraView& cam, unsigned long long seed,
                                   uint32_t frame, uint32_t W, uint32_t H, uint32_t max_depth, const NrcShadeArgs& nrc,
                                   float4* targets, DeviceStatus* status, int order, cudaStream_t st);

@@ -295,7 +295,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) train_kernel(TrainArgs a)
         {
             float in[8] = {}, other[8] = {};
             if (valid) {
-                const size_t rec = a.b.offset + (size_t)row * a.b.stride;
+                size_t rec = a.b.offset + (size_t)row * a.b.stride;
+                if (a.b.order) rec = __ldg(a.b.order + rec);
                 const Query q = load_query(a.b.queries + 4 * rec);
                 const float4 tg = __ldg(a.b.targets + rec);
                 target[0] = tg.x; target[1] = tg.y; target[2] = tg.z;

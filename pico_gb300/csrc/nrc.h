@@ -19,11 +19,13 @@ struct AdamStep {
     float c1, c2;          // 1 / (1 - beta1^t), 1 / (1 - beta2^t)
 };
 
-// One training batch: record j is queries[4 * (offset + j * stride)] with target targets[offset + j * stride].
+// One training batch: record j is queries[4 * r] with target targets[r], r = offset + j * stride or, with an order,
+// order[offset + j * stride].
 struct TrainBatch {
     const float4* queries;
     const float4* targets;
     uint32_t n, offset, stride;
+    const uint32_t* order = nullptr;
 };
 
 cudaError_t launch_encode(const GridGeometry& g, const __half2* table, const float4* queries, uint32_t n, float* out,

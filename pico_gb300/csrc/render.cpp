@@ -182,6 +182,9 @@ void for_cache_buffers(RenderBuffers& r, uint32_t group, uint32_t chunk_pix, uin
     f(r.nrc_q, (group == 1 ? std::max(records, terms) : records) * sizeof(pico_nrc_query));
     f(r.nrc_tp, records * 2 * sizeof(float4));
     f(r.nrc_tgt, records * sizeof(float4));
+    f(r.nrc_written, group * record_flags(rec_cap));
+    f(r.nrc_segments, group * record_segments(rec_cap) * sizeof(uint32_t));
+    f(r.nrc_order, records * sizeof(uint32_t));
     if (group > 1) f(r.nrc_term, terms * sizeof(pico_nrc_query));
     f(r.nrc_prev, slots * sizeof(float));
     f(r.nrc_count, 2 * kCancelSamplesPerBatch * sizeof(uint32_t));
@@ -236,7 +239,7 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
     const uint32_t max_depth = cfg->max_ray_depth;
     const uint32_t passes = c->cfg.warmup_frames + cfg->max_samples;
     const uint32_t rec_cap = (uint32_t)std::min<uint64_t>((uint64_t)ntrain * std::max(max_depth, 1u), 0xffffffffu);
-    // passes of a group: as many as 2^24 paths and 2^24 training records (112 bytes each, max_depth of them a training
+    // passes of a group: as many as 2^24 paths and 2^24 training records (117 bytes each, max_depth of them a training
     // path) hold, one when the image takes several chunks, fewer where the device's memory has no room for their state
     const uint32_t room = std::min(path_limit(ctx), 1u << 24);
     uint32_t group = std::max(1u, std::min({kCancelSamplesPerBatch, passes, (1u << 24) / std::max(rec_cap, 1u),
@@ -252,6 +255,9 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
     rec.capacity = rec_cap;
     rec.queries = as<float4>(r.nrc_q);
     rec.rec_tp = as<float4>(r.nrc_tp);
+    rec.written = as<uint8_t>(r.nrc_written);
+    rec.segments = as<uint32_t>(r.nrc_segments);
+    rec.order = as<uint32_t>(r.nrc_order);
     rec.count = as<uint32_t>(r.nrc_count);
     term.mode = kNrcTerminate;
     term.capacity = chunk_pix;
@@ -295,7 +301,7 @@ int render_with_cache(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, pico_gpu_n
         const uint32_t per = steps * ((nrec + steps * batch - 1) / (steps * batch));   // record stride
         for (uint32_t s = 0; s < steps && s < nrec; ++s) {
             const nrc::TrainBatch b{rec.queries + 4 * (size_t)k * rec_cap, as<float4>(r.nrc_tgt) + (size_t)k * rec_cap,
-                                    (nrec - s + per - 1) / per, s, per};
+                                    (nrec - s + per - 1) / per, s, per, rec.order + (size_t)k * rec_cap};
             const int status = nrc::train_step(c, b, true, st);
             if (status != PICO_OK) return status;
             c->render_stats[2] += 1;

@@ -13,9 +13,9 @@ struct RenderBuffers {
     pico::DeviceBuffer gn, gp, gd, ga, stats, out, tonemap;
     pico::DeviceBuffer hdr_pix, hdr_codes, hdr_lens, hdr_off, hdr_body;   // .hdr output: image, codes, their lengths
                                                                           // and places, the file's body
-    // radiance cache: training records' queries, throughput and payload, targets; terminal
-    // queries; previous roughness per path; entry counters
-    pico::DeviceBuffer nrc_q, nrc_tp, nrc_tgt, nrc_term, nrc_prev, nrc_count;
+    // radiance cache: training records' queries, throughput and payload, targets, which are written and their order;
+    // terminal queries; previous roughness per path; entry counters
+    pico::DeviceBuffer nrc_q, nrc_tp, nrc_tgt, nrc_written, nrc_segments, nrc_order, nrc_term, nrc_prev, nrc_count;
     size_t budget = ~size_t(0);   // pico_test_cache_budget
     // the host buffers this render's results will go to, populated once the device has its first work
     struct { void* p; size_t bytes; } results[3] = {};
@@ -34,7 +34,7 @@ struct RenderBuffers {
                                       &sorg, &sdir, &scontrib, &senergy, &q0, &q1, &sq, &counters, &pixels,
                                       &variance, &count, &taken, &done, &pix_list, &pix_list2, &plan, &gn, &gp, &gd,
                                       &ga, &stats,
-                                      &out, &tonemap, &hdr_pix, &hdr_codes, &hdr_lens, &hdr_off, &hdr_body, &nrc_q, &nrc_tp, &nrc_tgt, &nrc_term, &nrc_prev, &nrc_count})
+                                      &out, &tonemap, &hdr_pix, &hdr_codes, &hdr_lens, &hdr_off, &hdr_body, &nrc_q, &nrc_tp, &nrc_tgt, &nrc_written, &nrc_segments, &nrc_order, &nrc_term, &nrc_prev, &nrc_count})
             b->release();
     }
 };

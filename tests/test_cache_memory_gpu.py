@@ -14,10 +14,11 @@ W, H, DEPTH, SPP = 41, 30, 5, 20
 
 
 def _group_bytes(passes, paths):
-    """Path state, previous roughness, records (query, throughput and payload, target) and terminal queries."""
+    """Path state, previous roughness, records (query, throughput and payload, target, flag, place in the order) and
+    terminal queries."""
     slots, records, terms = passes * max(W * H, paths), passes * paths * DEPTH, passes * W * H
     queries = max(records, terms) if passes == 1 else records + terms
-    return slots * (208 + 4) + records * (32 + 16) + queries * 64 + 2048   # and two small arrays of counters
+    return slots * (208 + 4) + records * (32 + 16 + 5) + queries * 64 + 2048   # and some counters
 
 
 def _render(ctx, budget, paths, steps):
