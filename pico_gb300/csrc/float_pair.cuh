@@ -67,7 +67,7 @@ static __device__ __noinline__ float two_pi_times_double(float a) { return (floa
 __device__ __forceinline__ float two_pi_times(float a)
 {
     float out;
-    if (rounds(mul(P{kPi0, kPi1}, a), kRelPhi, out)) return 2.0f * out;
+    if (rounds(mul(P{kPi0, kPi1}, a), kRelPhi, out)) return copysignf(2.0f * out, a);   // the sum loses a zero's sign
     return two_pi_times_double(a);
 }
 
@@ -129,7 +129,7 @@ static __device__ __noinline__ float quotient_double(float e, float a, float c)
 __device__ __forceinline__ float quotient_by_pi(float e, float a, float c)
 {
     const P d = mul(mul(mul(P{kPi0, kPi1}, a), a), c);
-    if (e == 0.0f && d.h > 1e-12f && d.h < 1e12f) return 0.0f;
+    if (e == 0.0f && d.h > 1e-12f && d.h < 1e12f) return e;
     if (e > 1e-20f && e < 1e20f && d.h > 1e-12f && d.h < 1e12f) {
         const float i = __frcp_rn(d.h), q = __fmul_rn(e, i);
         const float res = __fmaf_rn(-q, d.l, __fmaf_rn(-q, d.h, e));
