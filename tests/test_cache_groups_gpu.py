@@ -42,3 +42,28 @@ def test_training_cache(ctx, spp, warmup):
     assert grouped[1:] == single[1:]
     assert grouped[1]["train_paths"] == 256 * (spp + warmup) and grouped[1]["train_steps"] > 0
     assert np.isfinite(grouped[0][0]).all() and (grouped[0][1] == spp).all()
+
+
+@pytest.mark.parametrize("spp", [5, 17, 33])
+def test_image_that_goes_on(ctx, spp):
+    """Some pixels finished, some with samples, some without: grouped and single passes take the same samples."""
+    gs, cam = ctx.upload(scenes.cornell_box()), scenes.cornell_camera(21, 13)
+    rng = np.random.default_rng(spp)
+    pix, var = (rng.random((13, 21, 3)).astype(np.float32) for _ in range(2))
+    count = rng.choice(np.array([0, 3, spp], np.uint32), (13, 21))
+    images = []
+    for limit in (0, 256):   # without a limit in groups; below, in chunks of at most 256 pixels, pass by pass
+        cache = RadianceCache(ctx, log2_table_size=12, seed=5, max_train_steps=0)
+        cache.attach()
+        ctx.set_path_limit(limit)
+        try:
+            images.append(gs.render(cam, 5, spp, seed=4, estimator=ESTIMATOR_RADIANCE_CACHE, pixels=pix.copy(),
+                                    sample_count=count.copy(), variance=var.copy()) + (cache.stats()["queries"],))
+        finally:
+            ctx.set_path_limit(0)
+            cache.free()
+    gs.free()
+    for a, b in zip(*images):
+        np.testing.assert_array_equal(a, b)
+    done = count == spp
+    assert 0 < done.sum() < done.size and (images[0][0][done] == pix[done]).all() and (images[0][1][~done] > spp - 1).all()

@@ -35,3 +35,12 @@ def test_images_in_turn(ctx, oracle):
     for h, w in ((40, 300), (3, 20), (17, 130)):
         img = rng.gamma(0.5, 2.0, (h, w, 3)).astype(np.float32)
         assert ctx.encode_hdr(img.reshape(-1, 3)[::-1].copy(), w, h) == oracle.hdr_file(img, w, h)
+
+
+@pytest.mark.parametrize("width", [7, 8, 32767, 32768])
+def test_widths_around_the_coded_ones(ctx, oracle, width):
+    """Rows of 8 to 32,767 pixels are run-length coded, the widest from 131,068 bytes of shared memory; others are not."""
+    rng = np.random.default_rng(width)
+    img = rng.choice(np.array([0.25, 0.5, 0.75], np.float32), (2, width, 3))
+    img[1, : width // 2] = rng.random((width // 2, 3))
+    assert ctx.encode_hdr(img.reshape(-1, 3)[::-1].copy(), width, 2) == oracle.hdr_file(img, width, 2)
