@@ -277,7 +277,10 @@ int pico_gpu_set_path_limit(pico_gpu_ctx* ctx, uint32_t max_paths);
  * samples each as fill the path state; otherwise every batch covers all pixels.
  * With a cancel flag (should_quit not NULL) it polls *should_quit before every
  * batch and a batch takes at most 16 samples per pixel: about 30-40 ms each for a
- * 1080p render on a GB300, which bounds how soon a cancel is seen. */
+ * 1080p render on a GB300, which bounds how soon a cancel is seen.  A radiance-cache
+ * render traces its passes (warm-up passes too) in groups of at most 16, with or without
+ * a flag, and polls before every group; one of several passes takes at most half of the device's free
+ * memory. */
 int pico_gpu_render(pico_gpu_ctx* ctx, const pico_gpu_scene* scene, const pico_camera* camera,
                     const pico_render_config* config, float* pixels_rgb, uint32_t* sample_count,
                     float* variance_rgb, const volatile int32_t* should_quit);

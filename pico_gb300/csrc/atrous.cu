@@ -23,7 +23,7 @@
 //          out = sum(w * c) / sum(w), evaluated with one exponential per tap
 //          (see the kernel).
 //
-// 1920 x 1080: 621 us before the records, cells and tiles below, 468 now.
+// 1920 x 1080: 621 us before the records, cells and tiles below, 452 now.
 //
 // The statistics are exact; the blend agrees with the reference's arithmetic to
 // about 1e-6 relative and keeps its NaN pattern.
@@ -326,8 +326,9 @@ static bool whole_footprints(uint32_t W, uint32_t H, int s)
 // a footprint row are split into even and odd columns so that a warp's loads hit consecutive records.
 //
 // Measured at 1920 x 1080 (start 92-98 us a level with its own tile kernel for spacings 1-4 and a direct one above):
-// 72-79 us a level at 60 % of the issue slots, 62 % of the shared-memory wavefronts and half of the FP32 pipe (whose
-// 36 us a level are the floor), 24 warps per SM waiting on shared-memory latency between.  Whole call: copies through
+// 68-77 us a level at 65 % of the issue slots, 61-67 % of the LSU wavefronts and half of the FP32 pipe (whose
+// 36 us a level are the floor), 24 warps per SM waiting on shared-memory latency between.  Whole call, while footprints
+// were copied whole: copies through
 // registers 595 us against 534 asynchronous; scalar differences 30 us more than packed ones; two rows per thread
 // (fewer reads, 20 warps) 528 against 509, three 605 against 534; 7 or 8 CTAs per SM (72 or 64 registers) 515 and 528;
 // tiles of 64 x 8, 32 x 16, 16 x 16 and 16 x 8 points 5, 5, 3 and 1 % slower.

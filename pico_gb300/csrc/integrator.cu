@@ -219,9 +219,10 @@ struct ExtendRays {
 // and, when sq is given, the shadow rays sq[0, *scount) the previous shade left
 // (they write disjoint path fields and both finish before the next shade), so a
 // depth pays one launch and one tail.  kThreads per CTA (64, 128 or 256): the
-// block shape batched renders tune; the register budget is the same for every
-// shape: 1152 threads (56 registers) per SM in the near-first order (walk_queue gives
-// the figures), and 896 threads in the reference's order, which spills more at 64.
+// block shape batched renders tune.  In the near-first order 64- and 128-thread CTAs
+// fill 1152 threads per SM (56 registers; walk_queue gives the figures), 256-thread
+// ones, of which that holds four, 1024 (63 registers); in the reference's order, which
+// spills more at 64, 896, 896 and 768 threads.
 // kCount: the same traversal, also adding its work (nodes, triangles, instance
 // entries) to `counters` (measurement only).
 template <int kOrder>

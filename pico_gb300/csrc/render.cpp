@@ -5,8 +5,8 @@
 // copied in, advanced by up to max_samples samples per pixel with the
 // reference's running mean / variance and early-exit rule, and copied back.
 // Pixels whose count already reaches max_samples are skipped, as the
-// reference's tile loop skips them.  Samples run as batches of at most 16M
-// paths (pixels x samples), each pixel's samples in order across batches; the
+// reference's tile loop skips them.  Samples run as batches of at most 2^26
+// paths (pixels x samples; fewer by pico_gpu_set_path_limit), each pixel's samples in order across batches; the
 // cancel flag is polled between batches.  When requested, the a-trous pass
 // then runs on the result and replaces it (Scene.cpp:212-234).
 // pico_gpu_render_device does the same on caller device buffers, asynchronously

@@ -416,7 +416,7 @@ __device__ __forceinline__ uint32_t tlas_rank(const SceneView& sc, uint32_t item
 }
 
 // The state of one near-first walk.  What the inner-node moves use lives in registers; what only the rarer moves
-// use lives in the walk's local memory, behind its stack (WalkMemory), which keeps the kernels free of spills.
+// use lives in the walk's local memory, behind its stack (WalkMemory), so that the loop's registers fit 56.
 //
 // The ray the node tests use is the world ray in the TLAS and the object-space
 // ray inside an instance, switched on entering and leaving an instance.  `limit`
@@ -728,7 +728,8 @@ __device__ __forceinline__ int nf_rare(NearFirstState& w, const SceneView& sc, u
 // those hand in their results together and take the next entries of the warp's
 // claim together, and the warp claims kClaim entries of the shared counter `work`
 // at a time.  What only the rarer moves use is kept in local memory, so that nine
-// CTAs of 128 threads (56 registers) fit an SM without spills.
+// CTAs of 128 threads (56 registers) fit an SM: without spills in the closest-hit
+// kernel, with 16 bytes stored and 12 loaded in the extension kernel.
 //
 // Measured on the closest-hit benchmark (16.8M rays, half primary, half bounces) and
 // the 1080p lit-field render, identical hits and images: one rare move per release,
